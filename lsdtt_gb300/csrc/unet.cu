@@ -56,8 +56,15 @@ __device__ __forceinline__ float bfr(float v) { return __bfloat162float(__float2
 // shuffle tree, then the block's warps in index order); one block then adds
 // the partials in a fixed tree (red_partials).
 constexpr int kRedBlocks = 152 * 4;
-// Pixel shares of one weight-gradient entry (k_conv_bwd_w's grid x).
-constexpr int kWgradBlocks = 64;
+// Shares of a layer's positions that its weight gradient is summed in
+// (k_bwd_w's grid x, times nine taps): enough blocks for every SM on the
+// small levels, and on large images no longer runs of FP32 additions.
+constexpr int kWgradMinSplits = 32, kWgradMaxSplits = 128;
+inline int wgrad_splits(std::int64_t positions)
+{
+    const std::int64_t s = positions / 2048;
+    return static_cast<int>(s < kWgradMinSplits ? kWgradMinSplits : (s > kWgradMaxSplits ? kWgradMaxSplits : s));
+}
 
 // The block's sum of v (all threads take part), valid in thread 0.
 __device__ __forceinline__ double block_sum_ordered(double v)
@@ -1429,132 +1436,416 @@ __global__ void k_loss_grad(const float* __restrict__ y, const float* __restrict
     go[i] = static_cast<float>(2.0 * (static_cast<double>(y[i]) - e[i]) / den * (*rms));
 }
 
-// Backward of a 3x3 conv w.r.t. its input: dX[q][ci] = sum_tap sum_co
-// g[q - off(tap)][co] * w[co][tap][ci]. g is [H][W][Cout] FP32 at the conv's
-// output resolution. With `up`, X was the nearest upsampling of a half-
-// resolution field, and the result is summed over each 2x2 block (written
-// at half resolution). With `pool_from` (encoder), dX is the gradient of the
-// pooled input, which is distributed /4 onto the full-resolution skip
-// gradient `acc_full` ([2H][2W][Cin], accumulated with +=) instead.
-__global__ void k_conv_bwd_data(int H, int W, int Cin, int Cout, int up, const float* __restrict__ g,
-                                const float* __restrict__ w, float* __restrict__ dx, int pool_to_full,
-                                float* __restrict__ acc_full)
+// Both gradients of a 3x3 convolution are sums over the same gathered output
+// gradient. For a position q of the layer's input X and a tap (dy, dx),
+//     GS_tap[q][co] = sum of g[p][co] over the output pixels p that read q
+//                     through that tap,
+// which is one pixel, q - (dy, dx), or with nearest upsampling the (up to)
+// four pixels p with (p + (dy, dx)) / 2 = q. Then
+//     dX[q][ci]       = sum over tap, co of GS_tap[q][co] w[co][tap][ci]
+//     gw[co][tap][ci] = sum over q of GS_tap[q][co] X[q][ci]
+//     gb[co]          = sum over q of GS_4[q][co],
+// two FP32 matrix products over tiles staged in shared memory. Summing the
+// four pixels of an upsampled position before the product takes a quarter of
+// the multiplications. What bounds them is the FP32 pipe (GB300's tensor
+// cores have no FP32 inputs). The forms that these replaced read every
+// operand from global memory once per multiplication: one gradient on
+// 512 x 512 took 8.70 ms with them (6.2 ms the weight gradients) and takes
+// 0.72 ms with these, forward pass included.
+//
+// GS of four consecutive output channels at position q of an Hq x Wq input.
+template <int CO, bool UP>
+__device__ __forceinline__ float4 bwd_gather(const float* __restrict__ g, int Hq, int Wq, int q, int c4, int dy, int dx)
+{
+    const int qy = q / Wq, qx = q - qy * Wq;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!UP)
+    {
+        const int py = qy - dy, px = qx - dx;
+        if (py >= 0 && py < Hq && px >= 0 && px < Wq)
+            v = *reinterpret_cast<const float4*>(g + (static_cast<std::int64_t>(py) * Wq + px) * CO + 4 * c4);
+        return v;
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+    {
+        const int py = 2 * qy - dy + (a >> 1), px = 2 * qx - dx + (a & 1);
+        if (py >= 0 && py < 2 * Hq && px >= 0 && px < 2 * Wq)
+        {
+            const float4 t =
+                *reinterpret_cast<const float4*>(g + (static_cast<std::int64_t>(py) * (2 * Wq) + px) * CO + 4 * c4);
+            v.x += t.x;
+            v.y += t.y;
+            v.z += t.z;
+            v.w += t.w;
+        }
+    }
+    return v;
+}
+
+// What becomes of dX (the gradient of the layer's input):
+//   kBwdSkip  the input was d = relu(pre) + skip: out = [pre > 0] dX, skip_out = dX;
+//   kBwdMask  the input was relu(act): out = [act > 0] dX;
+//   kBwdPool  the input was the 2x2 mean of act = relu(...), whose skip gradient is
+//             skip_in: at the four pixels out = [act > 0] (skip_in + dX / 4).
+enum : int { kBwdSkip = 0, kBwdMask = 1, kBwdPool = 2 };
+
+// dX over tiles of 4096 / CI positions, 256 threads with 4 positions x 4
+// channels each; the sum over (tap, co) goes in stages of 16 channels of one
+// tap, the next stage's global loads in flight while one is multiplied.
+template <int CI, int CO, bool UP, int MODE>
+__global__ void __launch_bounds__(256, 2) k_bwd_data(int Hq, int Wq, const float* __restrict__ g,
+                                                     const float* __restrict__ w,
+                                                     const __nv_bfloat16* __restrict__ act,
+                                                     const float* __restrict__ skip_in, float* __restrict__ out,
+                                                     float* __restrict__ skip_out)
 {
     LSDTT_COUNT();
-    const int Ho = up ? H / 2 : H, Wo = up ? W / 2 : W;  // resolution of the result
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<std::int64_t>(Ho) * Wo * Cin) return;
-    const int ci = static_cast<int>(i % Cin);
-    const std::int64_t q = i / Cin;
-    const int qy = static_cast<int>(q / Wo), qx = static_cast<int>(q % Wo);
-    float s = 0.f;
-    const int reps = up ? 4 : 1;
-    for (int sub = 0; sub < reps; ++sub)
+    constexpr int TQ = 4096 / CI, KC = 16;
+    constexpr int NG = TQ * KC / 4 / 256;          // float4 of GS per thread and stage
+    constexpr int NWt = KC * CI / 4;               // float4 of weights per stage
+    constexpr int STAGES = 9 * (CO / KC);
+    __shared__ __align__(16) float sG[KC][TQ], sW[KC][CI];
+    const int nq = Hq * Wq, q0 = blockIdx.x * TQ, tid = threadIdx.x;
+    const int tq = tid / (CI / 4), tc = tid % (CI / 4);
+    float4 rg[NG], rw = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto load = [&](int s) {
+        const int tap = s / (CO / KC), c0 = (s % (CO / KC)) * KC;
+#pragma unroll
+        for (int j = 0; j < NG; ++j)
+        {
+            const int i = tid + j * 256, q = q0 + i % TQ;
+            rg[j] = q < nq ? bwd_gather<CO, UP>(g, Hq, Wq, q, c0 / 4 + i / TQ, tap / 3 - 1, tap % 3 - 1)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (tid < NWt)
+            rw = *reinterpret_cast<const float4*>(
+                w + (static_cast<std::int64_t>(c0 + tid / (CI / 4)) * 9 + tap) * CI + 4 * (tid % (CI / 4)));
+    };
+    float acc[4][4] = {};
+    load(0);
+    for (int s = 0; s < STAGES; ++s)
     {
-        const int fy = up ? 2 * qy + (sub >> 1) : qy, fx = up ? 2 * qx + (sub & 1) : qx;
+        __syncthreads();  // the previous stage has been read
+#pragma unroll
+        for (int j = 0; j < NG; ++j)
+        {
+            const int i = tid + j * 256, q = i % TQ, k = 4 * (i / TQ);
+            sG[k][q] = rg[j].x;
+            sG[k + 1][q] = rg[j].y;
+            sG[k + 2][q] = rg[j].z;
+            sG[k + 3][q] = rg[j].w;
+        }
+        if (tid < NWt) *reinterpret_cast<float4*>(&sW[tid / (CI / 4)][4 * (tid % (CI / 4))]) = rw;
+        __syncthreads();
+        if (s + 1 < STAGES) load(s + 1);
+#pragma unroll
+        for (int k = 0; k < KC; ++k)
+        {
+            const float4 a = *reinterpret_cast<const float4*>(&sG[k][4 * tq]);
+            const float4 b = *reinterpret_cast<const float4*>(&sW[k][4 * tc]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+        const int q = q0 + 4 * tq + i;
+        if (q >= nq) continue;
+        auto masked = [&](std::int64_t at, float4 v) {
+            const __nv_bfloat162* m = reinterpret_cast<const __nv_bfloat162*>(act + at);
+            const float2 m0 = __bfloat1622float2(m[0]), m1 = __bfloat1622float2(m[1]);
+            *reinterpret_cast<float4*>(out + at) = make_float4(m0.x > 0.f ? v.x : 0.f, m0.y > 0.f ? v.y : 0.f,
+                                                               m1.x > 0.f ? v.z : 0.f, m1.y > 0.f ? v.w : 0.f);
+        };
+        const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        const std::int64_t at = static_cast<std::int64_t>(q) * CI + 4 * tc;
+        if (MODE == kBwdPool)
+        {
+            const int qy = q / Wq, qx = q - qy * Wq;
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+            {
+                const std::int64_t fa =
+                    (static_cast<std::int64_t>(2 * qy + (f >> 1)) * (2 * Wq) + 2 * qx + (f & 1)) * CI + 4 * tc;
+                const float4 k = *reinterpret_cast<const float4*>(skip_in + fa);
+                masked(fa, make_float4(k.x + v.x * 0.25f, k.y + v.y * 0.25f, k.z + v.z * 0.25f, k.w + v.w * 0.25f));
+            }
+        }
+        else
+        {
+            if (MODE == kBwdSkip) *reinterpret_cast<float4*>(skip_out + at) = v;
+            masked(at, v);
+        }
+    }
+}
+
+// Weight and bias gradients: block (split, tap) sums GS_tap x X over its
+// share of the positions, 8 x 8 (co, ci) accumulators a thread, the threads
+// that one copy of the (co, ci) plane leaves over taking other positions of
+// each 64-position stage (added at the end in a fixed tree). The splits'
+// partial sums go to part[split][parameter] and are added in split order by
+// k_bwd_w_sum, so the gradient has the same bits on every run.
+template <int CI, int CO, bool UP>
+__global__ void __launch_bounds__(256, 2) k_bwd_w(int Hq, int Wq, const float* __restrict__ g,
+                                                  const __nv_bfloat16* __restrict__ X, float* __restrict__ part,
+                                                  std::int64_t nparam, std::int64_t woff, std::int64_t boff)
+{
+    LSDTT_COUNT();
+    constexpr int TQ = 64;
+    constexpr int TPG = (CO / 8) * (CI / 8), GR = 256 / TPG;  // threads per copy, copies
+    constexpr int NG = TQ * CO / 4 / 256, NX = (TQ * CI / 8 + 255) / 256;
+    constexpr int kRed = 128 * 72;  // the tree's first step: half of the threads' 72 sums
+    constexpr int kStage = TQ * (CO + CI);
+    __shared__ __align__(16) float sm[kRed > kStage ? kRed : kStage];
+    float* sG = sm;
+    float* sX = sm + TQ * CO;
+    const int tid = threadIdx.x, grp = tid / TPG, t = tid % TPG;
+    const int co4 = 4 * (t / (CI / 8)), ci4 = 4 * (t % (CI / 8));  // channels co4.. and CO/2 + co4.., likewise ci
+    const int tap = blockIdx.y, dy = tap / 3 - 1, dx = tap % 3 - 1;
+    const int nq = Hq * Wq;
+    const int len = ((nq + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + TQ - 1) / TQ * TQ;
+    const int qa = min(nq, static_cast<int>(blockIdx.x) * len), qb = min(nq, qa + len);
+    float4 rg[NG];
+    uint4 rx[NX];
+    auto load = [&](int base) {
+#pragma unroll
+        for (int j = 0; j < NG; ++j)
+        {
+            const int i = tid + j * 256, q = base + i / (CO / 4);
+            rg[j] = q < qb ? bwd_gather<CO, UP>(g, Hq, Wq, q, i % (CO / 4), dy, dx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < NX; ++j)
+        {
+            const int i = tid + j * 256, q = base + i / (CI / 8);
+            rx[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (i < TQ * CI / 8 && q < qb)
+                rx[j] = *reinterpret_cast<const uint4*>(X + static_cast<std::int64_t>(q) * CI + 8 * (i % (CI / 8)));
+        }
+    };
+    float acc[8][8] = {}, bias[8] = {};
+    if (qa < qb) load(qa);
+    for (int base = qa; base < qb; base += TQ)
+    {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < NG; ++j) reinterpret_cast<float4*>(sG)[tid + j * 256] = rg[j];
+#pragma unroll
+        for (int j = 0; j < NX; ++j)
+        {
+            const int i = tid + j * 256;
+            if (i < TQ * CI / 8)
+            {
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rx[j]);
+                const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+                const float2 c = __bfloat1622float2(h[2]), d = __bfloat1622float2(h[3]);
+                reinterpret_cast<float4*>(sX)[2 * i] = make_float4(a.x, a.y, b.x, b.y);
+                reinterpret_cast<float4*>(sX)[2 * i + 1] = make_float4(c.x, c.y, d.x, d.y);
+            }
+        }
+        __syncthreads();
+        if (base + TQ < qb) load(base + TQ);
+#pragma unroll 2
+        for (int q = grp; q < TQ; q += GR)
+        {
+            const float4 a0 = *reinterpret_cast<const float4*>(sG + q * CO + co4);
+            const float4 a1 = *reinterpret_cast<const float4*>(sG + q * CO + CO / 2 + co4);
+            const float4 b0 = *reinterpret_cast<const float4*>(sX + q * CI + ci4);
+            const float4 b1 = *reinterpret_cast<const float4*>(sX + q * CI + CI / 2 + ci4);
+            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+            {
+                bias[i] += a[i];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            }
+        }
+    }
+    // the copies' sums, halves added until one is left
+    for (int n = GR; n > 1; n >>= 1)
+    {
+        const int half = n / 2 * TPG;
+        __syncthreads();
+        if (tid >= half && tid < 2 * half)
+        {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+            {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) sm[(8 * i + j) * half + tid - half] = acc[i][j];
+                sm[(64 + i) * half + tid - half] = bias[i];
+            }
+        }
+        __syncthreads();
+        if (tid < half)
+        {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+            {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] += sm[(8 * i + j) * half + tid];
+                bias[i] += sm[(64 + i) * half + tid];
+            }
+        }
+    }
+    if (tid >= TPG) return;
+    float* P = part + static_cast<std::int64_t>(blockIdx.x) * nparam;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+    {
+        const int co = (i < 4 ? 0 : CO / 2 - 4) + co4 + i;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            P[woff + (static_cast<std::int64_t>(co) * 9 + tap) * CI + (j < 4 ? 0 : CI / 2 - 4) + ci4 + j] = acc[i][j];
+        if (tap == 4 && ci4 == 0) P[boff + co] = bias[i];
+    }
+}
+
+// The one-channel layers' weight gradients: 16 channels of A at a pixel times
+// the nine shifted scalars of B. Layer 0 (kIn): A = g (FP32), B = x0 at p +
+// tap, gw[c][tap], gb[c] = sum g. Layer 7: A = d0 (bf16) at q, B = g at
+// q - tap, gw[tap][c], gb = sum g. A read-once pass bound by memory.
+template <bool kIn>
+__global__ void __launch_bounds__(256) k_bwd_w_one(int H, int W, const float* __restrict__ g,
+                                                   const __nv_bfloat16* __restrict__ X, float* __restrict__ part,
+                                                   std::int64_t nparam, std::int64_t woff, std::int64_t boff)
+{
+    LSDTT_COUNT();
+    __shared__ float red[8][160];
+    float acc[9][16] = {}, sum[kIn ? 16 : 1] = {};
+    const int n = H * W;
+    for (int p = static_cast<int>(blockIdx.x) * 256 + threadIdx.x; p < n; p += static_cast<int>(gridDim.x) * 256)
+    {
+        const int y = p / W, x = p - y * W;
+        float a[16], b[9];
+        if (kIn)
+        {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                const float4 v = reinterpret_cast<const float4*>(g + static_cast<std::int64_t>(p) * 16)[k];
+                a[4 * k] = v.x;
+                a[4 * k + 1] = v.y;
+                a[4 * k + 2] = v.z;
+                a[4 * k + 3] = v.w;
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+            {
+                const float2 v =
+                    __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(X + static_cast<std::int64_t>(p) * 16)[k]);
+                a[2 * k] = v.x;
+                a[2 * k + 1] = v.y;
+            }
+        }
+#pragma unroll
         for (int t = 0; t < 9; ++t)
         {
-            const int py = fy - (t / 3 - 1), px = fx - (t % 3 - 1);  // output pixel that reads (fy,fx) via tap t
-            if (py < 0 || py >= H || px < 0 || px >= W) continue;
-            const float* gp = g + (static_cast<std::int64_t>(py) * W + px) * Cout;
-            const float* wp = w + static_cast<std::int64_t>(t) * Cin + ci;
-            for (int co = 0; co < Cout; ++co) s += gp[co] * wp[static_cast<std::int64_t>(co) * 9 * Cin];
+            const int s = kIn ? 1 : -1, yy = y + s * (t / 3 - 1), xx = x + s * (t % 3 - 1);
+            const bool in = yy >= 0 && yy < H && xx >= 0 && xx < W;
+            const std::int64_t at = static_cast<std::int64_t>(yy) * W + xx;
+            b[t] = !in ? 0.f : (kIn ? __bfloat162float(X[at]) : g[at]);
         }
-    }
-    if (pool_to_full)
-    {
-        const int W2 = 2 * Wo;
-        const float v = s * 0.25f;
-        for (int sub = 0; sub < 4; ++sub)
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc[t][c] = fmaf(a[c], b[t], acc[t][c]);
+        if (kIn)
         {
-            const std::int64_t f = (static_cast<std::int64_t>(2 * qy + (sub >> 1)) * W2 + 2 * qx + (sub & 1)) * Cin + ci;
-            acc_full[f] += v;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) sum[c % (kIn ? 16 : 1)] += a[c];
         }
+        else
+            sum[0] += b[4];
     }
-    else
-        dx[i] = s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto put = [&](int k, float v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) red[warp][k] = v;
+    };
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) put(kIn ? c * 9 + t : t * 16 + c, acc[t][c]);
+#pragma unroll
+    for (int c = 0; c < (kIn ? 16 : 1); ++c) put(144 + c, sum[c]);
+    __syncthreads();
+    const int k = threadIdx.x;
+    if (k < 144 + (kIn ? 16 : 1))
+    {
+        float v = red[0][k];
+        for (int j = 1; j < 8; ++j) v += red[j][k];
+        part[static_cast<std::int64_t>(blockIdx.x) * nparam + (k < 144 ? woff + k : boff + k - 144)] = v;
+    }
 }
 
-// Weight/bias gradients of a 3x3 conv: gw[co][tap][ci] = sum_p g[p][co] *
-// X[p + off(tap)][ci], gb[co] = sum_p g[p][co]. Blocks (x, co * 9 + tap)
-// reduce over the x-th grid-strided share of the pixels and write their
-// partial sums to part[((co * 9 + tap) * (Cin + 1) + c) * gridDim.x + x]
-// (c = Cin: the bias term, tap 4 only); k_conv_bwd_w_sum adds the
-// gridDim.x partials of each entry in index order, so the gradient has the
-// same bits on every run. X is bf16 ([H][W][Cin], or half resolution with
-// `up`).
-__global__ void k_conv_bwd_w(int H, int W, int Cin, int Cout, int up, const float* __restrict__ g,
-                             const __nv_bfloat16* __restrict__ X, float* __restrict__ part)
+// Gradient of the output layer's input (1 -> 16 channels through the nine
+// taps), with the kBwdSkip outputs.
+__global__ void __launch_bounds__(256) k_bwd_data_out(int H, int W, const float* __restrict__ g,
+                                                      const float* __restrict__ w, const __nv_bfloat16* __restrict__ pre,
+                                                      float* __restrict__ out, float* __restrict__ skip_out)
 {
     LSDTT_COUNT();
-    extern __shared__ float red[];  // [Cin + 1][32]
-    const int co = blockIdx.y / 9, t = blockIdx.y % 9;
-    const int Win = up ? W / 2 : W;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    float acc_c[64 + 1];
-    for (int c = 0; c <= Cin; ++c) acc_c[c] = 0.f;
-    const std::int64_t npix = static_cast<std::int64_t>(H) * W;
-    for (std::int64_t p = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < npix;
-         p += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
-    {
-        const float gv = g[p * Cout + co];
-        if (gv == 0.f) continue;
-        if (t == 4) acc_c[Cin] += gv;
-        const int py = static_cast<int>(p / W) + t / 3 - 1, px = static_cast<int>(p % W) + t % 3 - 1;
-        if (py < 0 || py >= H || px < 0 || px >= W) continue;
-        const __nv_bfloat16* xp = X + (static_cast<std::int64_t>(up ? py >> 1 : py) * Win + (up ? px >> 1 : px)) * Cin;
-        for (int c = 0; c < Cin; ++c) acc_c[c] += gv * __bfloat162float(xp[c]);
-    }
-    for (int c = 0; c <= Cin; ++c)
-    {
-        float v = acc_c[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[c * 32 + warp] = v;
-    }
+    __shared__ __align__(16) float sw[144];
+    if (threadIdx.x < 144) sw[threadIdx.x] = w[threadIdx.x];
     __syncthreads();
-    if (threadIdx.x <= Cin)
+    // four threads a pixel, four channels each
+    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * 256 + threadIdx.x;
+    if (i >= static_cast<std::int64_t>(H) * W * 4) return;
+    const std::int64_t p = i >> 2;
+    const int c4 = 4 * static_cast<int>(i & 3);
+    const int y = static_cast<int>(p / W), x = static_cast<int>(p - static_cast<std::int64_t>(y) * W);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
     {
-        float v = 0.f;
-        for (int k = 0; k < nw; ++k) v += red[threadIdx.x * 32 + k];
-        part[(static_cast<std::int64_t>(blockIdx.y) * (Cin + 1) + threadIdx.x) * gridDim.x + blockIdx.x] = v;
+        const int yy = y - (t / 3 - 1), xx = x - (t % 3 - 1);
+        if (yy < 0 || yy >= H || xx < 0 || xx >= W) continue;
+        const float v = g[static_cast<std::int64_t>(yy) * W + xx];
+        const float4 k = *reinterpret_cast<const float4*>(sw + 16 * t + c4);
+        s.x = fmaf(v, k.x, s.x);
+        s.y = fmaf(v, k.y, s.y);
+        s.z = fmaf(v, k.z, s.z);
+        s.w = fmaf(v, k.w, s.w);
     }
+    const std::int64_t at = p * 16 + c4;
+    *reinterpret_cast<float4*>(skip_out + at) = s;
+    const __nv_bfloat162* m = reinterpret_cast<const __nv_bfloat162*>(pre + at);
+    const float2 m0 = __bfloat1622float2(m[0]), m1 = __bfloat1622float2(m[1]);
+    *reinterpret_cast<float4*>(out + at) = make_float4(m0.x > 0.f ? s.x : 0.f, m0.y > 0.f ? s.y : 0.f,
+                                                       m1.x > 0.f ? s.z : 0.f, m1.y > 0.f ? s.w : 0.f);
 }
 
-// gw / gb from the partials of k_conv_bwd_w (nx per entry), in index order.
-__global__ void k_conv_bwd_w_sum(int Cin, int Cout, int nx, const float* __restrict__ part, float* __restrict__ gw,
-                                 float* __restrict__ gb)
+// Every parameter's gradient from its layer's partial sums, in split order.
+struct WgradSplits
+{
+    std::int64_t woff[kLayers + 1], boff[kLayers + 1];
+    int splits[kLayers];
+};
+
+__global__ void __launch_bounds__(256) k_bwd_w_sum(std::int64_t nparam, WgradSplits S, const float* __restrict__ part,
+                                                   float* __restrict__ g)
 {
     LSDTT_COUNT();
     const std::int64_t j = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j >= static_cast<std::int64_t>(Cout) * 9 * (Cin + 1)) return;
-    const int y = static_cast<int>(j / (Cin + 1)), c = static_cast<int>(j % (Cin + 1));
-    const float* p = part + j * nx;
+    if (j >= nparam) return;
+    const std::int64_t* off = j < S.woff[kLayers] ? S.woff : S.boff;
+    int l = 0;
+    while (l + 1 < kLayers && j >= off[l + 1]) ++l;
     float v = 0.f;
-    for (int k = 0; k < nx; ++k) v += p[k];
-    if (c < Cin) gw[static_cast<std::int64_t>(y) * Cin + c] = v;
-    else if (y % 9 == 4) gb[y / 9] = v;
-}
-
-// Decoder split: ga = gd * (pre > 0); gskip += gd.
-__global__ void k_relu_skip_bwd(std::int64_t n, const float* __restrict__ gd, const __nv_bfloat16* __restrict__ pre,
-                                float* __restrict__ ga, float* __restrict__ gskip)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = gd[i];
-    ga[i] = __bfloat162float(pre[i]) > 0.f ? v : 0.f;
-    gskip[i] += v;
-}
-
-// Encoder: g = gsum * (act > 0) (act = relu output, bf16).
-__global__ void k_relu_mask(std::int64_t n, const float* __restrict__ gsum, const __nv_bfloat16* __restrict__ act,
-                            float* __restrict__ g)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    g[i] = __bfloat162float(act[i]) > 0.f ? gsum[i] : 0.f;
+#pragma unroll 8
+    for (int k = 0; k < S.splits[l]; ++k) v += part[k * nparam + j];
+    g[j] = v;
 }
 
 __global__ void k_adam(std::int64_t n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
@@ -1637,8 +1928,8 @@ struct lsdtt_gpu_unet
     double* hacc = nullptr;
     // training-only buffers (decoder pre-activations a0..a2 above, FP32
     // backward scratch), allocated by the first gradient evaluation
-    float *gA = nullptr, *gB = nullptr, *ge0 = nullptr, *ge1 = nullptr, *ge2 = nullptr, *ge3 = nullptr;
-    float* gwpart = nullptr;  // weight-gradient partials [Cout * 9][Cin + 1][kWgradBlocks] of the widest layer
+    float *gA = nullptr, *gB = nullptr, *ge0 = nullptr, *ge1 = nullptr, *ge2 = nullptr;
+    float* gwpart = nullptr;  // weight-gradient partial sums [wgrad_splits of the capacity][nparam]
 };
 
 namespace
@@ -1895,55 +2186,51 @@ cudaError_t unet_forward(lsdtt_gpu_unet* U, const float* r, int H, int W, cudaSt
 cudaError_t unet_backward(lsdtt_gpu_unet* U, const float* e, int H, int W, cudaStream_t st)
 {
     const std::int64_t n = static_cast<std::int64_t>(H) * W;
-    // every weight and bias entry is assigned by k_conv_bwd_w_sum below
+    // every weight and bias entry is assigned by k_bwd_w_sum below
     k_loss_sums<<<kRedBlocks, 256, 0, st>>>(U->y, e, n, U->part + kRedBlocks);
     red_partials<<<2, 256, 0, st>>>(U->part + kRedBlocks, kRedBlocks, U->acc + 1);
     k_loss_grad<<<grid_blocks(n, 256), 256, 0, st>>>(U->y, e, n, U->acc + 1, U->rms, U->go);
     const float* wr = U->wr;
-    auto bw = [&](int l, int h, int w, int up, const float* g, const __nv_bfloat16* X) {
-        const int ci = layer_cin(l), co = layer_cout(l);
-        const dim3 grid(kWgradBlocks, co * 9);
-        k_conv_bwd_w<<<grid, 256, sizeof(float) * (ci + 1) * 32, st>>>(h, w, ci, co, up, g, X, U->gwpart);
-        const std::int64_t entries = static_cast<std::int64_t>(co) * 9 * (ci + 1);
-        k_conv_bwd_w_sum<<<grid_blocks(entries, 256), 256, 0, st>>>(ci, co, kWgradBlocks, U->gwpart,
-                                                                     U->g + U->woff[l], U->g + U->boff[l]);
-    };
-    // out layer (16 -> 1): input d0 at H x W
-    bw(7, H, W, 0, U->go, U->d0);
-    k_conv_bwd_data<<<grid_blocks(n * 16, 256), 256, 0, st>>>(H, W, 16, 1, 0, U->go, wr + U->woff[7], U->gA, 0,
-                                                              nullptr);
-    // ge0 starts as the skip gradient from d0; dec0: d0 = relu(a0) + e0
-    cudaMemsetAsync(U->ge0, 0, sizeof(float) * n * 16, st);
-    k_relu_skip_bwd<<<grid_blocks(n * 16, 256), 256, 0, st>>>(n * 16, U->gA, U->a0, U->gB, U->ge0);
-    bw(6, H, W, 1, U->gB, U->d1);  // input of dec0 is up(d1)
-    const std::int64_t n1 = n / 4, n2 = n / 16, n3 = n / 64;
-    k_conv_bwd_data<<<grid_blocks(n1 * 32, 256), 256, 0, st>>>(H, W, 32, 16, 1, U->gB, wr + U->woff[6], U->gA, 0,
-                                                               nullptr);  // gd1 (half res) in gA
-    cudaMemsetAsync(U->ge1, 0, sizeof(float) * n1 * 32, st);
-    k_relu_skip_bwd<<<grid_blocks(n1 * 32, 256), 256, 0, st>>>(n1 * 32, U->gA, U->a1, U->gB, U->ge1);
-    bw(5, H / 2, W / 2, 1, U->gB, U->d2);
-    k_conv_bwd_data<<<grid_blocks(n2 * 64, 256), 256, 0, st>>>(H / 2, W / 2, 64, 32, 1, U->gB, wr + U->woff[5], U->gA,
-                                                               0, nullptr);  // gd2
-    cudaMemsetAsync(U->ge2, 0, sizeof(float) * n2 * 64, st);
-    k_relu_skip_bwd<<<grid_blocks(n2 * 64, 256), 256, 0, st>>>(n2 * 64, U->gA, U->a2, U->gB, U->ge2);
-    bw(4, H / 4, W / 4, 1, U->gB, U->e3);
-    k_conv_bwd_data<<<grid_blocks(n3 * 64, 256), 256, 0, st>>>(H / 4, W / 4, 64, 64, 1, U->gB, wr + U->woff[4],
-                                                               U->ge3, 0, nullptr);  // ge3 (1/8 res)
-    // encoder 3: e3 = relu(conv(p2)); p2 = pool(e2)
-    k_relu_mask<<<grid_blocks(n3 * 64, 256), 256, 0, st>>>(n3 * 64, U->ge3, U->e3, U->gB);
-    bw(3, H / 8, W / 8, 0, U->gB, U->p2);
-    k_conv_bwd_data<<<grid_blocks(n3 * 64, 256), 256, 0, st>>>(H / 8, W / 8, 64, 64, 0, U->gB, wr + U->woff[3],
-                                                               nullptr, 1, U->ge2);
-    k_relu_mask<<<grid_blocks(n2 * 64, 256), 256, 0, st>>>(n2 * 64, U->ge2, U->e2, U->gB);
-    bw(2, H / 4, W / 4, 0, U->gB, U->p1);
-    k_conv_bwd_data<<<grid_blocks(n2 * 32, 256), 256, 0, st>>>(H / 4, W / 4, 32, 64, 0, U->gB, wr + U->woff[2],
-                                                               nullptr, 1, U->ge1);
-    k_relu_mask<<<grid_blocks(n1 * 32, 256), 256, 0, st>>>(n1 * 32, U->ge1, U->e1, U->gB);
-    bw(1, H / 2, W / 2, 0, U->gB, U->p0);
-    k_conv_bwd_data<<<grid_blocks(n1 * 16, 256), 256, 0, st>>>(H / 2, W / 2, 16, 32, 0, U->gB, wr + U->woff[1],
-                                                               nullptr, 1, U->ge0);
-    k_relu_mask<<<grid_blocks(n * 16, 256), 256, 0, st>>>(n * 16, U->ge0, U->e0, U->gB);
-    bw(0, H, W, 0, U->gB, U->x0);
+    WgradSplits S{};
+    for (int l = 0; l <= kLayers; ++l)
+    {
+        S.woff[l] = U->woff[l];
+        S.boff[l] = U->boff[l];
+    }
+    // weight gradient of layer l over the positions of its input (h x w)
+#define LSDTT_BWD_W(l, h, w, UP, g, X)                                                                                \
+    do                                                                                                                 \
+    {                                                                                                                  \
+        S.splits[l] = wgrad_splits(static_cast<std::int64_t>(h) * (w));                                                \
+        k_bwd_w<layer_cin(l), layer_cout(l), UP><<<dim3(S.splits[l], 9), 256, 0, st>>>(                                \
+            h, w, g, X, U->gwpart, U->nparam, U->woff[l], U->boff[l]);                                                 \
+    } while (0)
+#define LSDTT_BWD_DATA(l, h, w, UP, MODE, g, act, skip_in, out, skip_out)                                             \
+    k_bwd_data<layer_cin(l), layer_cout(l), UP, MODE>                                                                 \
+        <<<grid_blocks(static_cast<std::int64_t>(h) * (w), 4096 / layer_cin(l)), 256, 0, st>>>(                       \
+            h, w, g, wr + U->woff[l], act, skip_in, out, skip_out)
+    S.splits[0] = S.splits[7] = wgrad_splits(n);
+    // output layer (16 -> 1) on d0 = relu(a0) + e0
+    k_bwd_w_one<false><<<S.splits[7], 256, 0, st>>>(H, W, U->go, U->d0, U->gwpart, U->nparam, U->woff[7], U->boff[7]);
+    k_bwd_data_out<<<grid_blocks(n * 4, 256), 256, 0, st>>>(H, W, U->go, wr + U->woff[7], U->a0, U->gB, U->ge0);
+    // decoder: inputs up(d1), up(d2), up(e3)
+    LSDTT_BWD_W(6, H / 2, W / 2, true, U->gB, U->d1);
+    LSDTT_BWD_DATA(6, H / 2, W / 2, true, kBwdSkip, U->gB, U->a1, nullptr, U->gA, U->ge1);
+    LSDTT_BWD_W(5, H / 4, W / 4, true, U->gA, U->d2);
+    LSDTT_BWD_DATA(5, H / 4, W / 4, true, kBwdSkip, U->gA, U->a2, nullptr, U->gB, U->ge2);
+    LSDTT_BWD_W(4, H / 8, W / 8, true, U->gB, U->e3);
+    LSDTT_BWD_DATA(4, H / 8, W / 8, true, kBwdMask, U->gB, U->e3, nullptr, U->gA, nullptr);
+    // encoder: inputs p2 = pool(e2), p1 = pool(e1), p0 = pool(e0), x0
+    LSDTT_BWD_W(3, H / 8, W / 8, false, U->gA, U->p2);
+    LSDTT_BWD_DATA(3, H / 8, W / 8, false, kBwdPool, U->gA, U->e2, U->ge2, U->gB, nullptr);
+    LSDTT_BWD_W(2, H / 4, W / 4, false, U->gB, U->p1);
+    LSDTT_BWD_DATA(2, H / 4, W / 4, false, kBwdPool, U->gB, U->e1, U->ge1, U->gA, nullptr);
+    LSDTT_BWD_W(1, H / 2, W / 2, false, U->gA, U->p0);
+    LSDTT_BWD_DATA(1, H / 2, W / 2, false, kBwdPool, U->gA, U->e0, U->ge0, U->gB, nullptr);
+    k_bwd_w_one<true><<<S.splits[0], 256, 0, st>>>(H, W, U->gB, U->x0, U->gwpart, U->nparam, U->woff[0], U->boff[0]);
+#undef LSDTT_BWD_W
+#undef LSDTT_BWD_DATA
+    k_bwd_w_sum<<<grid_blocks(U->nparam, 256), 256, 0, st>>>(U->nparam, S, U->gwpart, U->g);
     return cudaGetLastError();
 }
 
@@ -2072,7 +2359,7 @@ int lsdtt_gpu_unet_destroy(lsdtt_gpu_unet* U)
     if (!U) return LSDTT_GPU_OK;
     void* ptrs[] = {U->w, U->wr, U->wb, U->g, U->m, U->v, U->x0, U->e0, U->a0, U->d0, U->p0, U->e1, U->a1, U->d1, U->p1,
                     U->e2, U->a2, U->d2, U->p2, U->e3, U->y, U->go, U->rms, U->acc, U->part, U->gA, U->gB, U->ge0,
-                    U->ge1, U->ge2, U->ge3, U->gwpart, U->d_err};
+                    U->ge1, U->ge2, U->gwpart, U->d_err};
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(U->hacc);
     delete U;
@@ -2151,15 +2438,15 @@ int lsdtt_gpu_unet_loss_grad(lsdtt_gpu_unet* U, const float* r_dev, const float*
         if (e == cudaSuccess) e = ualloc(&U->ge0, px0 * 16);
         if (e == cudaSuccess) e = ualloc(&U->ge1, level_px(U, 1) * 32);
         if (e == cudaSuccess) e = ualloc(&U->ge2, level_px(U, 2) * 64);
-        if (e == cudaSuccess) e = ualloc(&U->ge3, level_px(U, 3) * 64);
-        // widest weight-gradient reduction: Cout 64 x 9 taps x (Cin 64 + bias)
-        if (e == cudaSuccess) e = ualloc(&U->gwpart, static_cast<std::size_t>(64) * 9 * 65 * kWgradBlocks);
+        // partial sums of every parameter's gradient, one set per split
+        if (e == cudaSuccess)
+            e = ualloc(&U->gwpart, static_cast<std::size_t>(U->nparam) * static_cast<std::size_t>(wgrad_splits(px0)));
         if (e != cudaSuccess)
         {
-            void* bufs[] = {U->a0, U->a1, U->a2, U->gA, U->gB, U->ge0, U->ge1, U->ge2, U->ge3, U->gwpart};
+            void* bufs[] = {U->a0, U->a1, U->a2, U->gA, U->gB, U->ge0, U->ge1, U->ge2, U->gwpart};
             for (void* b : bufs) cudaFree(b);
             U->a0 = U->a1 = U->a2 = nullptr;
-            U->gA = U->gB = U->ge0 = U->ge1 = U->ge2 = U->ge3 = nullptr;
+            U->gA = U->gB = U->ge0 = U->ge1 = U->ge2 = nullptr;
             U->gwpart = nullptr;
             return cuda_fail(e, "lsdtt_gpu_unet_loss_grad");
         }
