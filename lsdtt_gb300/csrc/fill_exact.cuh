@@ -83,8 +83,8 @@ inline std::size_t ex_bytes(std::int64_t N, int M, std::int64_t fifo_total)
     for (std::size_t w : {16, 16, 8, 8, 8, 4, 4, 4, 4, 1, 1, 1, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4})
         b += ex_round(w * n);
     b += ex_round(8 * (n + 2));  // global heap
-    // block replay: cst, ev, te, te_st, te_k, mk_c, dc, dc2, dk, dk2, sc, sk
-    for (std::size_t w : {4, 16, 16, 4, 1, 4, 4, 4, 4, 4, 4, 4}) b += ex_round(w * n);
+    // block replay: ev, te, te_st, te_k, mk_c, dc, dc2, dk, dk2, sc, sk
+    for (std::size_t w : {16, 16, 4, 1, 4, 4, 4, 4, 4, 4, 4}) b += ex_round(w * n);
     b += 2 * ex_round(4 * static_cast<std::size_t>(kSwLv) * n);  // lc, lk
     b += ex_round(4 * m);  // chain order
     b += ex_round(4 * m);
@@ -122,7 +122,7 @@ inline bool ex_carve(Scratch& ws, std::int64_t N, int M, std::int64_t fifo_total
     B.stamp = ws.take<std::uint32_t>(n);
     B.ghk = ws.take<std::uint64_t>(n + 2);
     B.gfq = ws.take<std::uint64_t>(static_cast<std::size_t>(fifo_total) + 1);
-    B.sw.cst = ws.take<std::uint32_t>(n);
+    B.sw.cst = B.rec ? reinterpret_cast<std::uint32_t*>(B.rec) + 3 : nullptr;  // no buffer of its own
     B.sw.ev = ws.take<SwEv>(n);
     B.sw.te = ws.take<SwTe>(n);
     B.sw.te_st = ws.take<std::uint32_t>(n);
@@ -205,7 +205,7 @@ __global__ void ex_prep(const ExMember* __restrict__ mem, const std::uint16_t* _
                 mn = fminf(mn, fj);
                 if (zi <= f && zj == fj && fj == f) pour = true;
             }
-            B.rec[i] = make_float4(zi, f, (kind[i] == 2) ? -INFINITY : mn, 1.0f);
+            B.rec[i] = make_float4(zi, f, (kind[i] == 2) ? -INFINITY : mn, __uint_as_float(1u));
             has_pour = pour;
             pour_key = hi | float_order_key(f);
         }
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kSwThreads) ex_chain(const ExMember* __restric
     SweepBufs sb = B.sw;
     {
         const std::int64_t o = M.base;
-        sb.cst += o;
+        sb.cst += 4 * o;
         sb.ev += o;
         sb.te += o;
         sb.te_st += o;
@@ -589,7 +589,7 @@ inline cudaError_t ex_run(const ExMember* mem, const std::uint16_t* blk_member, 
     if (e == cudaSuccess) e = cudaMemsetAsync(B.diff, 0, sizeof(int) * (static_cast<std::size_t>(N) + 1), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(B.stamp, 0, sizeof(std::uint32_t) * static_cast<std::size_t>(N), st);
     // the block replay's stamps and counters start from zero on every run
-    for (std::uint32_t* a : {B.sw.cst, B.sw.mk_c, B.sw.te_st})
+    for (std::uint32_t* a : {B.sw.mk_c, B.sw.te_st})
         if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, sizeof(std::uint32_t) * static_cast<std::size_t>(N), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(B.sw.ev, 0, sizeof(SwEv) * static_cast<std::size_t>(N), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(B.sw_ctr, 0, sizeof(std::uint32_t) * M, st);

@@ -72,7 +72,8 @@ __host__ __device__ __forceinline__ float float_from_order_key(std::uint32_t k)
 // One grid (or one ensemble member) as the window replay sees it; every
 // pointer and cell index is member-local. Per cell one 16-byte record
 // {z, F0 (epsilon-0 fill), mnb (min F0 over valid neighbours; -inf for
-// seeds, +inf for cells never queued), class (0 invalid or NaN, 1 valid)};
+// seeds, +inf for cells never queued), state word (bits: 0 invalid or NaN, 1
+// valid, above: queued by a block replay's window)};
 // per sorted position {F0, mnb, cell, -} over the valid cells by
 // (F0, index): one load gives a replay all it needs of a cell.
 struct WinGrid
@@ -471,7 +472,7 @@ __device__ WinResult win_replay(const WinGrid& G, int w, const WinStore& s, std:
         }
         // open: valid, not popped before the window (F0 >= S), not queued
         // at its start (mnb >= S)
-        if (j != kWinNone && !(q.w != 0.0f && q.y >= S && !(q.z < S))) j = kWinNone;
+        if (j != kWinNone && !(__float_as_uint(q.w) != 0u && q.y >= S && !(q.z < S))) j = kWinNone;
         const float zj = q.x;
         // a neighbour reached twice through a periodic wrap counts once
         if (dedupe)
