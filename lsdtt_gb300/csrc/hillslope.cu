@@ -28,162 +28,408 @@ namespace lsdtt_gb300
 namespace
 {
 
-// DOF flag, Jacobi inverse diagonal and b = -F (linear law) in one pass.
-__global__ void hs_setup(Hs H, const std::uint8_t* __restrict__ mask, const std::uint8_t* __restrict__ chan,
-                         const float* __restrict__ z, const float* __restrict__ zn, std::uint8_t* __restrict__ dof,
-                         float* __restrict__ inv_diag, float* __restrict__ b, double* __restrict__ acc)
+// ---- grid-wide sums --------------------------------------------------------
+// Each block writes one FP64 partial per quantity; the block that finishes
+// last adds them in index order and forms the solver's next coefficient
+// there. Against one FP64 atomic a block on a single address (0.76 ns each at
+// the L2) or a one-block kernel after every pass (4.5 us of its own) this
+// leaves about a microsecond, and the sums are the same on every run.
+// Within a block a sum is carried in two FP32 words (error-free additions,
+// about 48 bits): a warp's FP64 addition holds this part's FP64 pipe for 16
+// cycles, and ten of them a warp and quantity cost 6 us of a 16 us pass over a
+// million cells.
+struct Sum2
 {
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const std::int64_t n = static_cast<std::int64_t>(H.nr) * H.nc;
-    double bb = 0.0, fin = 0.0;
-    if (i < n)
+    float h = 0.0f, l = 0.0f;
+    __device__ __forceinline__ void add(float v)
     {
-        const int r = static_cast<int>(i / H.nc), c = static_cast<int>(i % H.nc);
-        const bool is_dof = mask[i] && !(chan && chan[i]) && !hs_dirichlet_edge(H, r, c);
-        // 3: a fast cell for the tiled operator (interior, its four
-        // neighbours in the grid and DOFs themselves), 1: any other DOF
-        bool fast = false;
-        if (is_dof && r > 0 && r < H.nr - 1 && c > 0 && c < H.nc - 1)
-        {
-            auto nb_dof = [&](int rr, int cc) {
-                const std::int64_t j = static_cast<std::int64_t>(rr) * H.nc + cc;
-                return mask[j] && !(chan && chan[j]) && !hs_dirichlet_edge(H, rr, cc);
-            };
-            fast = nb_dof(r - 1, c) && nb_dof(r, c + 1) && nb_dof(r + 1, c) && nb_dof(r, c - 1);
-        }
-        dof[i] = is_dof ? (fast ? 3 : 1) : 0;
-        if (is_dof)
-        {
-            const double zp = z[i];
-            double flux = 0.0;
-            int nf = 0;
+        const float t = h + v, q = t - h;
+        l += (h - (t - q)) + (v - q);
+        h = t;
+    }
+};
+
+template <int K>
+__device__ __forceinline__ void block_partials(Sum2 (&v)[K], double* __restrict__ part, unsigned nblk)
+{
+    __shared__ Sum2 sh_part[K][8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto fold = [&](Sum2& a, int from) {
 #pragma unroll
-            for (int f = 0; f < 4; ++f)
-            {
-                const std::int64_t j = hs_nb(H, mask, r, c, kDr[f], kDc[f]);
-                // sum_f alpha_f * S_n,f * h with S_n = (z_nb - z_P)/h (operator_cpu.hpp:299-305)
-                flux += static_cast<double>(z[j]) - zp;
-                nf += (j != i) ? 1 : 0;
-            }
-            double F = -H.U - H.DA * flux;
-            F += H.inv_dt * (zp - static_cast<double>(zn[i]));
-            b[i] = static_cast<float>(-F);
-            inv_diag[i] = static_cast<float>(1.0 / (H.inv_dt + H.DA * nf));
-            bb = F * F;
-            fin = fabs(F);
-        }
-        else
+        for (int o = from; o > 0; o >>= 1)
         {
-            b[i] = 0.0f;
-            inv_diag[i] = 0.0f;
+            const float h = __shfl_down_sync(0xffffffffu, a.h, o), l = __shfl_down_sync(0xffffffffu, a.l, o);
+            a.add(h);
+            a.l += l;
         }
-    }
-    block_atomic_add(&acc[0], bb);
-    block_atomic_max_nonneg(&acc[1], fin);
-}
-
-// x = 0, r = b, zz = M^-1 r, p = zz, acc[2] = r.zz
-__global__ void hs_cg_init(std::int64_t n, const float* __restrict__ b, const float* __restrict__ inv_diag,
-                           float* __restrict__ x, float* __restrict__ r, float* __restrict__ p, double* __restrict__ acc)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    double rz = 0.0;
-    if (i < n)
-    {
-        const float ri = b[i];
-        const float zi = ri * inv_diag[i];
-        x[i] = 0.0f;
-        r[i] = ri;
-        p[i] = zi;
-        rz = static_cast<double>(ri) * zi;
-    }
-    block_atomic_add(&acc[2], rz);
-}
-
-// Ap = J p (matrix-free) fused with p.Ap  -> acc_it[0]
-__global__ void hs_apply(Hs H, const std::uint8_t* __restrict__ mask, const std::uint8_t* __restrict__ dof,
-                         const float* __restrict__ p, float* __restrict__ Ap, double* __restrict__ acc_it)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const std::int64_t n = static_cast<std::int64_t>(H.nr) * H.nc;
-    // FP32 difference form inv_dt p_P + (D/h^2) sum_f (p_P - [nb DOF] p_nb):
-    // no large terms cancel, and no FP64 per cell.
-    const float inv_dt = static_cast<float>(H.inv_dt), DA = static_cast<float>(H.DA);
-    float pap = 0.0f;
-    if (i < n)
-    {
-        float v = 0.0f;
-        if (dof[i])
-        {
-            const int r = static_cast<int>(i / H.nc);
-            const int c = static_cast<int>(i - static_cast<std::int64_t>(r) * H.nc);
-            const float pi = p[i];
-            float s = 0.0f;
+    };
 #pragma unroll
-            for (int f = 0; f < 4; ++f)
-            {
-                const std::int64_t j = hs_nb(H, mask, r, c, kDr[f], kDc[f]);
-                if (j == i) continue;
-                s += pi - (dof[j] ? p[j] : 0.0f);
-            }
-            v = inv_dt * pi + DA * s;
-            pap = pi * v;
-        }
-        Ap[i] = v;
-    }
-    block_atomic_add_f(&acc_it[0], pap);
-}
-
-// alpha = rz/pAp; x += alpha p; r -= alpha Ap; zz = M^-1 r; acc_it[1] = r.zz, acc_it[2] = r.r
-__global__ void hs_update(std::int64_t n, const double* __restrict__ rz_prev, const double* __restrict__ acc_it,
-                          const float* __restrict__ inv_diag, const float* __restrict__ p, const float* __restrict__ Ap,
-                          float* __restrict__ x, float* __restrict__ r, float* __restrict__ zz,
-                          double* __restrict__ acc_out)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    // alpha once per block: a per-thread FP64 division costs more than the
-    // kernel's memory traffic on this part.
-    __shared__ float s_alpha;
-    if (threadIdx.x == 0)
+    for (int k = 0; k < K; ++k)
     {
-        const double pap = acc_it[0];
-        s_alpha = (pap > 0.0) ? static_cast<float>(*rz_prev / pap) : 0.0f;
+        fold(v[k], 16);
+        if (lane == 0) sh_part[k][w] = v[k];
     }
     __syncthreads();
-    const float alpha = s_alpha;
-    float rz = 0.0f, rr = 0.0f;
-    if (i < n)
+    if (w < K)
     {
-        x[i] += alpha * p[i];
-        const float ri = r[i] - alpha * Ap[i];
-        r[i] = ri;
-        const float zi = ri * inv_diag[i];
-        zz[i] = zi;
-        rz = ri * zi;
-        rr = ri * ri;
+        Sum2 a;
+        if (lane < 8) a = sh_part[w][lane];
+        fold(a, 4);
+        if (lane == 0)
+        {
+            part[static_cast<std::size_t>(w) * nblk + blockIdx.x] = static_cast<double>(a.h) + static_cast<double>(a.l);
+            __threadfence();
+        }
     }
-    block_atomic_add_f(&acc_out[1], rz);
-    block_atomic_add_f(&acc_out[2], rr);
 }
 
-// beta = rz_new / rz_old; p = zz + beta p
-__global__ void hs_direction(std::int64_t n, const double* __restrict__ rz_old, const double* __restrict__ rz_new,
-                             const float* __restrict__ zz, float* __restrict__ p)
+// After block_partials: true in the last block to arrive (every thread of it).
+__device__ __forceinline__ bool last_block(unsigned* __restrict__ arrived, unsigned nblk)
+{
+    __shared__ bool sh_last;
+    __syncthreads();
+    if (threadIdx.x == 0) sh_last = atomicInc(arrived, nblk - 1) == nblk - 1;  // wraps to 0 for the next pass
+    __syncthreads();
+    if (sh_last) __threadfence();
+    return sh_last;
+}
+
+// The last block's totals of K quantities (thread 0 holds them).
+template <int K>
+__device__ __forceinline__ void total_partials(const double* __restrict__ part, unsigned nblk, double (&out)[K])
+{
+    __shared__ double sh_tot[K][8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+    {
+        double s = 0.0;
+        for (unsigned b = threadIdx.x; b < nblk; b += blockDim.x)
+            s += __ldcg(part + static_cast<std::size_t>(k) * nblk + b);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) sh_tot[k][w] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+        {
+            out[k] = sh_tot[k][0];
+            for (int j = 1; j < static_cast<int>(blockDim.x >> 5); ++j) out[k] += sh_tot[k][j];
+        }
+}
+
+// A cell's class: 0 not a degree of freedom; else bit 0 set, bit 1 "fast"
+// (interior, its four neighbours in the grid and DOFs themselves), bits 2-5
+// the faces N, E, S, W that lead to another cell.
+__device__ __forceinline__ unsigned hs_class(const Hs& H, const std::uint8_t* __restrict__ mask,
+                                             const std::uint8_t* __restrict__ chan, int r, int c)
+{
+    auto is_dof = [&](int rr, int cc) {
+        const std::int64_t j = static_cast<std::int64_t>(rr) * H.nc + cc;
+        return mask[j] && !(chan && chan[j]) && !hs_dirichlet_edge(H, rr, cc);
+    };
+    if (!is_dof(r, c)) return 0u;
+    const std::int64_t i = static_cast<std::int64_t>(r) * H.nc + c;
+    const bool fast = r > 0 && r < H.nr - 1 && c > 0 && c < H.nc - 1 && is_dof(r - 1, c) && is_dof(r, c + 1) &&
+                      is_dof(r + 1, c) && is_dof(r, c - 1);
+    if (fast) return 1u | 2u | (15u << 2);
+    unsigned faces = 0;
+#pragma unroll
+    for (int f = 0; f < 4; ++f) faces |= (hs_nb(H, mask, r, c, kDr[f], kDc[f]) != i ? 4u : 0u) << f;
+    return 1u | faces;
+}
+
+// The class plane for the Roering solver.
+__global__ void hs_dofs(Hs H, const std::uint8_t* __restrict__ mask, const std::uint8_t* __restrict__ chan,
+                        std::uint8_t* __restrict__ dof)
 {
     LSDTT_COUNT();
     const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    __shared__ float s_beta;
+    if (i >= static_cast<std::int64_t>(H.nr) * H.nc) return;
+    const int r = static_cast<int>(i / H.nc), c = static_cast<int>(i - static_cast<std::int64_t>(r) * H.nc);
+    dof[i] = static_cast<std::uint8_t>(hs_class(H, mask, chan, r, c));
+}
+
+// ---- linear step -------------------------------------------------------------
+// Jacobi-PCG in two passes an iteration:
+//   hsl_direction  p = D^-1 r + beta p_old, stored; sum p.(A p), then alpha
+//   hsl_update     A p again from p; x += alpha p, r -= alpha A p; sums
+//                  r.D^-1 r and r.r, then beta and the convergence test
+// D^-1 is one of five values (a cell's class says how many faces it has), so
+// neither it nor D^-1 r nor A p is an array: 34 bytes a cell and iteration.
+//
+// A warp walks a strip 32 columns wide (30 of them its own, the outer lanes
+// the halo) down RW rows: north and south neighbours are its registers, east
+// and west a shuffle, and all loads of the strip are issued before the first
+// is used. The halo wraps where the edge does, a cell's class says which of
+// its faces lead to another cell, and p is 0 at a cell that is not a DOF, so
+// every cell takes the same path: resolving an edge cell's neighbours one by
+// one (mask, class, values: three dependent loads each) made the warps of the
+// east and west edges the longest by far, 47 us of a pass on 2048 x 2051. The
+// passes now take 24 and 33 us there (about 8 of each the grid-wide sum's
+// chain of fence, arrival and last block) where the three untiled passes they
+// replace took 162: a solve of 80 iterations 14.2 -> 5.3 ms.
+constexpr int kHslTC = 128;  // columns of a set-up block
+
+struct Strip
+{
+    int r0, c;     // first own row, this lane's column
+    bool own;      // the lane's column is the warp's own (and on the grid)
+    bool any;      // the strip exists
+    int nr, up, dn;  // rows read as row -1 and row nr (-1: none)
+    __device__ Strip(const Hs& H, int rw)
+    {
+        const int nc = H.nc;
+        nr = H.nr;
+        up = H.bn == 'p' ? nr - 1 : -1;
+        dn = H.bs == 'p' ? 0 : -1;
+        const int ns = (nc + 29) / 30;
+        const int g = static_cast<int>(blockIdx.x) * 8 + static_cast<int>(threadIdx.x >> 5);
+        const int lane = threadIdx.x & 31;
+        r0 = g / ns * rw;
+        c = g % ns * 30 - 1 + lane;
+        any = r0 < nr;
+        own = any && lane >= 1 && lane <= 30 && c < nc;
+        // the halo column a wrapped edge reads
+        if (c == -1) c = H.bw == 'p' ? nc - 1 : -1;
+        else if (c == nc) c = H.be == 'p' ? 0 : -1;
+        else if (c > nc) c = -1;
+    }
+    // Row k - 1 of the strip as it is read (-1: none).
+    __device__ __forceinline__ int row(int k) const
+    {
+        const int r = r0 - 1 + k;
+        return !any || c < 0 ? -1 : (r < 0 ? up : (r < nr ? r : (r == nr ? dn : -1)));
+    }
+};
+
+// Blocks of a strip pass.
+inline unsigned strip_blocks(int nr, int nc, int rw)
+{
+    const std::int64_t g = static_cast<std::int64_t>((nc + 29) / 30) * ((nr + rw - 1) / rw);
+    return static_cast<unsigned>((g + 7) / 8);
+}
+// Rows a warp walks: 16 where that leaves every SM 32 warps (two halo rows in
+// 18 loaded, not two in 10), else 8.
+inline bool strip_long(int nr, int nc) { return strip_blocks(nr, nc, 16) >= 4 * 152; }
+
+struct HsState
+{
+    double bb, rz, rr, rel, finf;
+    float alpha, beta;
+    int iters, done;
+    unsigned arrived, pad;
+};
+
+struct HslArgs
+{
+    Hs H;
+    float inv_dt, DA;
+    float invd[5];  // 1 / (1/dt + faces * D/h^2)
+    const std::uint8_t* mask;
+    const std::uint8_t* cls;
+    HsState* S;
+    double* part;
+    double rel_tol;
+    int max_iter;
+};
+
+__device__ __forceinline__ float hsl_invd(const HslArgs& A, unsigned cl)
+{
+    const int f = __popc(cl >> 2);
+    return !(cl & 1u) ? 0.0f : (f == 4 ? A.invd[4] : (f == 3 ? A.invd[3] : (f == 2 ? A.invd[2] : (f == 1 ? A.invd[1] : A.invd[0]))));
+}
+
+// Classes, b = -F (F = -(D/h^2) sum_f (z_nb - z_P), its sum and product carried
+// in two FP32 words each, so b is rounded once as from FP64), r = b, x = 0;
+// ||b||^2, r.D^-1 r, max |F|.
+__global__ void __launch_bounds__(256) hsl_setup(HslArgs A, float DA_lo, const std::uint8_t* __restrict__ chan,
+                                                 const float* __restrict__ z, std::uint8_t* __restrict__ cls,
+                                                 float* __restrict__ r, float* __restrict__ x)
+{
+    LSDTT_COUNT();
+    const Hs& H = A.H;
+    const int ntx = (H.nc + kHslTC - 1) / kHslTC;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int row = static_cast<int>(blockIdx.x / ntx) * 8 + w, c0 = static_cast<int>(blockIdx.x % ntx) * kHslTC;
+    Sum2 v[2];
+    float mh = 0.0f, ml = 0.0f;  // largest |b| before its rounding
+    if (row < H.nr)
+    {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            const int c = c0 + 32 * k + lane;
+            if (c >= H.nc) continue;
+            const std::int64_t i = static_cast<std::int64_t>(row) * H.nc + c;
+            const unsigned cl = hs_class(H, A.mask, chan, row, c);
+            cls[i] = static_cast<std::uint8_t>(cl);
+            x[i] = 0.0f;
+            float b = 0.0f;
+            if (cl)
+            {
+                const float zp = z[i];
+                float sh = 0.0f, sl = 0.0f;
+#pragma unroll
+                for (int f = 0; f < 4; ++f)
+                {
+                    const std::int64_t j = (cl & 2u) ? i + static_cast<std::int64_t>(kDr[f]) * H.nc + kDc[f]
+                                                     : hs_nb(H, A.mask, row, c, kDr[f], kDc[f]);
+                    // (d, e) = z_nb - z_P exactly, then added to (sh, sl)
+                    const float zj = z[j], d = zj - zp, t = d - zj, e = (zj - (d - t)) + (-zp - t);
+                    const float u = sh + d, q = u - sh;
+                    sl += ((sh - (u - q)) + (d - q)) + e;
+                    sh = u;
+                }
+                const float ph = A.DA * sh;
+                const float pl = fmaf(A.DA, sh, -ph) + (A.DA * sl + DA_lo * sh);
+                b = ph + pl;
+                const float bl = (ph - b) + pl;
+                const float ah = fabsf(b), al = b < 0.0f ? -bl : bl;
+                if (ah > mh || (ah == mh && al > ml))
+                {
+                    mh = ah;
+                    ml = al;
+                }
+                v[0].add(b * b);
+                v[1].add(b * (b * hsl_invd(A, cl)));
+            }
+            r[i] = b;
+        }
+    }
+    const unsigned nblk = gridDim.x;
+    block_atomic_max_nonneg(&A.S->finf, static_cast<double>(mh) + static_cast<double>(ml));
+    block_partials<2>(v, A.part, nblk);
+    if (!last_block(&A.S->arrived, nblk)) return;
+    double t[2];
+    total_partials<2>(A.part, nblk, t);
     if (threadIdx.x == 0)
     {
-        const double ro = *rz_old;
-        s_beta = (ro > 0.0) ? static_cast<float>(*rz_new / ro) : 0.0f;
+        A.S->bb = t[0];
+        A.S->rz = t[1];
+        A.S->beta = 0.0f;
+        A.S->done = t[0] == 0.0 ? 1 : 0;
     }
-    __syncthreads();
-    if (i < n) p[i] = zz[i] + s_beta * p[i];
+}
+
+// A p at a cell from its own and its neighbours' p (faces in the order N, E,
+// S, W).
+__device__ __forceinline__ float hsl_op(const HslArgs& A, float pi, float pn, float pe, float ps, float pw, unsigned cl)
+{
+    float s = 0.0f;
+    s += (cl & 4u) ? pi - pn : 0.0f;
+    s += (cl & 8u) ? pi - pe : 0.0f;
+    s += (cl & 16u) ? pi - ps : 0.0f;
+    s += (cl & 32u) ? pi - pw : 0.0f;
+    return A.inv_dt * pi + A.DA * s;
+}
+
+template <int RW, bool kFirst>
+__global__ void __launch_bounds__(256) hsl_direction(HslArgs A, const float* __restrict__ r,
+                                                     const float* __restrict__ p_old, float* __restrict__ p)
+{
+    LSDTT_COUNT();
+    if (A.S->done) return;
+    const int nr = A.H.nr, nc = A.H.nc;
+    const Strip t(A.H, RW);
+    const float beta = A.S->beta;
+    float rv[RW + 2], pv[RW + 2];
+    unsigned cl[RW + 2];
+#pragma unroll
+    for (int k = 0; k < RW + 2; ++k)
+    {
+        const int row = t.row(k);
+        const bool in = row >= 0;
+        const std::int64_t i = static_cast<std::int64_t>(row) * nc + t.c;
+        cl[k] = in ? A.cls[i] : 0u;
+        rv[k] = in ? r[i] : 0.0f;
+        pv[k] = (in && !kFirst) ? p_old[i] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < RW + 2; ++k)
+    {
+        const float d = hsl_invd(A, cl[k]) * rv[k];
+        pv[k] = kFirst ? d : d + beta * pv[k];
+    }
+    Sum2 v[1];
+#pragma unroll
+    for (int k = 1; k <= RW; ++k)
+    {
+        const float pe = __shfl_down_sync(0xffffffffu, pv[k], 1), pw = __shfl_up_sync(0xffffffffu, pv[k], 1);
+        if (t.own && t.r0 - 1 + k < nr)
+        {
+            p[static_cast<std::int64_t>(t.r0 - 1 + k) * nc + t.c] = pv[k];
+            if (cl[k]) v[0].add(pv[k] * hsl_op(A, pv[k], pv[k - 1], pe, pv[k + 1], pw, cl[k]));
+        }
+    }
+    const unsigned nblk = gridDim.x;
+    block_partials<1>(v, A.part, nblk);
+    if (!last_block(&A.S->arrived, nblk)) return;
+    double s[1];
+    total_partials<1>(A.part, nblk, s);
+    if (threadIdx.x == 0) A.S->alpha = s[0] > 0.0 ? static_cast<float>(A.S->rz / s[0]) : 0.0f;
+}
+
+template <int RW>
+__global__ void __launch_bounds__(256) hsl_update(HslArgs A, const float* __restrict__ p, float* __restrict__ x,
+                                                  float* __restrict__ r)
+{
+    LSDTT_COUNT();
+    if (A.S->done) return;
+    const int nr = A.H.nr, nc = A.H.nc;
+    const Strip t(A.H, RW);
+    const float alpha = A.S->alpha;
+    float pv[RW + 2], xv[RW], rv[RW];
+    unsigned cl[RW];
+#pragma unroll
+    for (int k = 0; k < RW + 2; ++k)
+    {
+        const int row = t.row(k);
+        const std::int64_t i = static_cast<std::int64_t>(row) * nc + t.c;
+        pv[k] = row >= 0 ? p[i] : 0.0f;
+        if (k >= 1 && k <= RW)
+        {
+            const bool in = t.own && t.r0 - 1 + k < nr;
+            cl[k - 1] = in ? A.cls[i] : 0u;
+            xv[k - 1] = in ? x[i] : 0.0f;
+            rv[k - 1] = in ? r[i] : 0.0f;
+        }
+    }
+    Sum2 v[2];
+#pragma unroll
+    for (int k = 1; k <= RW; ++k)
+    {
+        const float pe = __shfl_down_sync(0xffffffffu, pv[k], 1), pw = __shfl_up_sync(0xffffffffu, pv[k], 1);
+        const unsigned c1 = cl[k - 1];
+        if (c1)
+        {
+            const std::int64_t i = static_cast<std::int64_t>(t.r0 - 1 + k) * nc + t.c;
+            x[i] = xv[k - 1] + alpha * pv[k];
+            const float ri = rv[k - 1] - alpha * hsl_op(A, pv[k], pv[k - 1], pe, pv[k + 1], pw, c1);
+            r[i] = ri;
+            v[0].add(ri * (ri * hsl_invd(A, c1)));
+            v[1].add(ri * ri);
+        }
+    }
+    const unsigned nblk = gridDim.x;
+    block_partials<2>(v, A.part, nblk);
+    if (!last_block(&A.S->arrived, nblk)) return;
+    double s[2];
+    total_partials<2>(A.part, nblk, s);
+    if (threadIdx.x == 0)
+    {
+        HsState& S = *A.S;
+        S.beta = S.rz > 0.0 ? static_cast<float>(s[0] / S.rz) : 0.0f;
+        S.rz = s[0];
+        S.rr = s[1];
+        const int it = ++S.iters;
+        if (it % 4 == 0 || it >= A.max_iter)
+        {
+            S.rel = sqrt(s[1]) / sqrt(S.bb);
+            if (S.rel <= A.rel_tol || it >= A.max_iter) S.done = 1;
+        }
+    }
 }
 
 __global__ void hs_finish(std::int64_t n, const std::uint8_t* __restrict__ dof, const float* __restrict__ z,
@@ -192,7 +438,7 @@ __global__ void hs_finish(std::int64_t n, const std::uint8_t* __restrict__ dof, 
     LSDTT_COUNT();
     const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    out[i] = dof[i] ? static_cast<float>(static_cast<double>(z[i]) + static_cast<double>(x[i])) : z[i];
+    out[i] = dof[i] ? __fadd_rn(z[i], x[i]) : z[i];  // the exact sum, rounded once
 }
 
 }  // namespace
@@ -224,77 +470,74 @@ extern "C" int lsdtt_gpu_hillslope_linear_implicit(const lsdtt_gpu_grid* grid, c
     H.DA = static_cast<double>(D) / (h * h);
     H.inv_dt = 1.0 / static_cast<double>(dt);
     H.U = 0.0;
-    // Scratch: dof u8, inv_diag, bvec, x, r, p, zz, Ap (f32) + reductions.
+    // Scratch: x, r, two directions (f32), classes u8, partials, state.
+    const int kMaxIt = max_iter > 0 ? max_iter : 1000;
+    const std::size_t fbytes = (sizeof(float) * static_cast<std::size_t>(n) + 255) & ~std::size_t(255);
+    const std::size_t cbytes = (static_cast<std::size_t>(n) + 255) & ~std::size_t(255);
+    const int ntx = (H.nc + kHslTC - 1) / kHslTC;
+    const unsigned tiles8 = static_cast<unsigned>(ntx) * static_cast<unsigned>((H.nr + 7) / 8);
+    const bool tall = strip_long(H.nr, H.nc);
+    const unsigned tiles = strip_blocks(H.nr, H.nc, tall ? 16 : 8);
+    const std::size_t need = 4 * fbytes + cbytes + sizeof(double) * 2 * static_cast<std::size_t>(std::max(tiles8, tiles)) + 1024;
     char* base = nullptr;
-    const std::size_t fbytes = sizeof(float) * static_cast<std::size_t>(n);
-    const std::size_t need = 7 * ((fbytes + 255) & ~std::size_t(255)) + n + 4096;
     cudaError_t e = cudaMallocAsync(&base, need, st);
     if (e != cudaSuccess) return cuda_fail(e, "lsdtt_gpu_hillslope_linear_implicit");
-    auto carve = [&](std::size_t bytes) {
-        char* p = base;
-        base += (bytes + 255) & ~std::size_t(255);
-        return p;
-    };
-    char* const start = base;
-    float* invd = reinterpret_cast<float*>(carve(fbytes));
-    float* bv = reinterpret_cast<float*>(carve(fbytes));
-    float* x = reinterpret_cast<float*>(carve(fbytes));
-    float* r = reinterpret_cast<float*>(carve(fbytes));
-    float* p = reinterpret_cast<float*>(carve(fbytes));
-    float* zz = reinterpret_cast<float*>(carve(fbytes));
-    float* Ap = reinterpret_cast<float*>(carve(fbytes));
-    std::uint8_t* dof = reinterpret_cast<std::uint8_t*>(carve(static_cast<std::size_t>(n)));
-    // acc[0] ||b||^2, acc[1] ||F||inf, acc[2] r.z (initial), then per
-    // iteration k a triple at acc[4 + 3k]: pAp, r.z, r.r
-    const int kMaxIt = max_iter > 0 ? max_iter : 1000;
-    double* acc = nullptr;
-    double* hacc = nullptr;
-    e = cudaMallocAsync(&acc, sizeof(double) * (4 + 3 * (kMaxIt + 1)), st);
-    if (e == cudaSuccess) e = cudaMallocHost(&hacc, sizeof(double) * 8);
-    if (e != cudaSuccess)
-    {
-        cudaFreeAsync(start, st);
-        return cuda_fail(e, "lsdtt_gpu_hillslope_linear_implicit");
-    }
-    cudaMemsetAsync(acc, 0, sizeof(double) * (4 + 3 * (kMaxIt + 1)), st);
+    float* x = reinterpret_cast<float*>(base);
+    float* r = reinterpret_cast<float*>(base + fbytes);
+    float* pbuf[2] = {reinterpret_cast<float*>(base + 2 * fbytes), reinterpret_cast<float*>(base + 3 * fbytes)};
+    std::uint8_t* cls = reinterpret_cast<std::uint8_t*>(base + 4 * fbytes);
+    HslArgs A{};
+    A.S = reinterpret_cast<HsState*>(base + 4 * fbytes + cbytes);
+    A.part = reinterpret_cast<double*>(base + 4 * fbytes + cbytes + 512);
+    A.H = H;
+    A.inv_dt = static_cast<float>(H.inv_dt);
+    A.DA = static_cast<float>(H.DA);
+    for (int f = 0; f < 5; ++f) A.invd[f] = static_cast<float>(1.0 / (H.inv_dt + H.DA * f));
+    A.mask = mask_dev;
+    A.cls = cls;
+    A.rel_tol = rel_tol;
+    A.max_iter = kMaxIt;
+    cudaMemsetAsync(A.S, 0, sizeof(HsState), st);
     const unsigned nb = grid_blocks(n, 256);
-    hs_setup<<<nb, 256, 0, st>>>(H, mask_dev, is_channel_dev, z_dev, z_dev, dof, invd, bv, acc);
-    hs_cg_init<<<nb, 256, 0, st>>>(n, bv, invd, x, r, p, acc);
-    cudaMemcpyAsync(hacc, acc, sizeof(double) * 3, cudaMemcpyDeviceToHost, st);
-    e = cudaStreamSynchronize(st);
-    int it = 0;
-    double rel = 0.0;
-    const double bnorm = e == cudaSuccess ? std::sqrt(hacc[0]) : 0.0;
-    const double finf0 = hacc[1];
-    bool converged = bnorm == 0.0;
-    const int kCheck = 4;
-    while (e == cudaSuccess && !converged && it < kMaxIt)
+    hsl_setup<<<tiles8, 256, 0, st>>>(A, static_cast<float>(H.DA - static_cast<double>(A.DA)), is_channel_dev, z_dev, cls,
+                                      r, x);
+    // Iterations in batches, each followed by one read of the state; a batch
+    // launched past convergence returns at once.
+    HsState S{};
+    int queued = 0, batch = 4;
+    while (e == cudaSuccess)
     {
-        const int batch = std::min(kCheck, kMaxIt - it);
-        for (int k = 0; k < batch; ++k, ++it)
+        for (int k = 0; k < batch && queued < kMaxIt; ++k, ++queued)
         {
-            double* cur = acc + 4 + 3 * it;
-            const double* rz_prev = (it == 0) ? acc + 2 : acc + 4 + 3 * (it - 1) + 1;
-            // Algorithmic bytes (fused 3-kernel PCG iteration: 44 B/cell): Ap = A p with p.Ap, 8 B/cell.
-            LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
-                        (hs_apply<<<nb, 256, 0, st>>>(H, mask_dev, dof, p, Ap, cur)));
-            hs_update<<<nb, 256, 0, st>>>(n, rz_prev, cur, invd, p, Ap, x, r, zz, cur);
-            hs_direction<<<nb, 256, 0, st>>>(n, rz_prev, cur + 1, zz, p);
+            const float* po = pbuf[(queued + 1) & 1];
+            float* p = pbuf[queued & 1];
+            // Algorithmic bytes: residual 4, class 1, old direction 4 in, direction 4 out.
+            LSDTT_TIMED("hillslope_apply", 13.0 * static_cast<double>(n), st, ({
+                            if (tall)
+                            {
+                                if (queued == 0) hsl_direction<16, true><<<tiles, 256, 0, st>>>(A, r, po, p);
+                                else hsl_direction<16, false><<<tiles, 256, 0, st>>>(A, r, po, p);
+                            }
+                            else if (queued == 0) hsl_direction<8, true><<<tiles, 256, 0, st>>>(A, r, po, p);
+                            else hsl_direction<8, false><<<tiles, 256, 0, st>>>(A, r, po, p);
+                        }));
+            if (tall) hsl_update<16><<<tiles, 256, 0, st>>>(A, p, x, r);
+            else hsl_update<8><<<tiles, 256, 0, st>>>(A, p, x, r);
         }
-        cudaMemcpyAsync(hacc, acc + 4 + 3 * (it - 1), sizeof(double) * 3, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&S, A.S, sizeof(S), cudaMemcpyDeviceToHost, st);
         e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) break;
-        rel = std::sqrt(hacc[2]) / bnorm;
-        converged = rel <= rel_tol;
+        if (S.done || queued >= kMaxIt) break;
+        batch = std::min(16, batch + 4);
     }
+    const int it = S.iters;
+    const double rel = S.rel, finf0 = S.finf;
+    const bool converged = S.bb == 0.0 || (it > 0 && rel <= rel_tol);
     if (e == cudaSuccess)
     {
-        hs_finish<<<nb, 256, 0, st>>>(n, dof, z_dev, x, z_out_dev);
+        hs_finish<<<nb, 256, 0, st>>>(n, cls, z_dev, x, z_out_dev);
         e = cudaStreamSynchronize(st);
     }
-    cudaFreeAsync(start, st);
-    cudaFreeAsync(acc, st);
-    cudaFreeHost(hacc);
+    cudaFreeAsync(base, st);
     if (e != cudaSuccess) return cuda_fail(e, "lsdtt_gpu_hillslope_linear_implicit");
     if (report)
     {
@@ -528,7 +771,7 @@ __device__ __forceinline__ void block_store_d(double v, double* dst)
 // Operator value at a cell of the tile: inv_dt x_P + (D/h^2) sum_f alpha_f
 // (x_P - [nb DOF] x_nb) in FP32 (the difference form keeps the operator
 // symmetric: alpha is a property of the face), the faces summed in the order
-// N, E, S, W on both paths. Fast cells (dof 3: interior, all four neighbours
+// N, E, S, W on both paths. Fast cells (class bit 1: interior, all four neighbours
 // DOFs) read the neighbours from the tile; other DOFs resolve them by the
 // boundary rules and `xg` (the global value of a cell).
 template <class XG>
@@ -541,7 +784,7 @@ __device__ __forceinline__ float hs_op_cell(const HsN& P, float inv_dt, float DA
     if (kd == 0) return 0.0f;
     const float4 a = alpha[i];
     float s = 0.0f;
-    if (kd == 3)
+    if (kd & 2)
     {
         s += a.x * (xi - sx[lr - 1][lc]);
         s += a.y * (xi - sx[lr][lc + 1]);
@@ -585,53 +828,88 @@ __device__ __forceinline__ void hs_stage_tile(float (&sx)[kHsTR + 2][132], int n
     __syncthreads();
 }
 
-// Ap = A p over one tile per block, part[tile] = p.Ap (FP32 within each
-// 32-cell warp row, FP64 beyond). With kFuse the direction update of the
-// previous iteration, p = z + beta p (beta = scal[1]), is formed while
-// staging: p_src is read, p_dst written.
-template <bool kFuse>
+// The PCG loops' state beside the coefficients scal[0] (alpha), scal[1] (beta).
+struct HsnLoop
+{
+    double rel;
+    int iters, done;
+    unsigned arrived, pad;
+};
+
+// Ap = A p and p.Ap into *pap_out, from which the last block forms
+// alpha = *rz / p.Ap (scal[0]), over strips as in the linear step (10.9 us at
+// 1024 x 1000; 21 us over 128 x 32 tiles, whose edge warps resolved each
+// neighbour by loads and of which there were only 256). With kFuse
+// the direction update of the previous iteration, p = z + beta p
+// (beta = scal[1]), is formed on the way: p_src is read, p_dst written.
+template <bool kFuse, int RW>
 __global__ void __launch_bounds__(256) hsn_apply_t(HsN P, float inv_dt, float DA, const std::uint8_t* __restrict__ mask,
                                                    const std::uint8_t* __restrict__ dof,
-                                                   const float4* __restrict__ alpha, const float* __restrict__ scal,
+                                                   const float4* __restrict__ alpha, float* __restrict__ scal,
                                                    const float* __restrict__ zz, const float* __restrict__ p_src,
                                                    float* __restrict__ p_dst, float* __restrict__ Ap,
-                                                   double* __restrict__ part)
+                                                   double* __restrict__ part, HsnLoop* __restrict__ L,
+                                                   const double* __restrict__ rz, double* __restrict__ pap_out)
 {
     LSDTT_COUNT();
-    __shared__ float sx[kHsTR + 2][132];
+    if (L->done) return;
     const int nr = P.H.nr, nc = P.H.nc;
-    const int ntx = (nc + kHsTC - 1) / kHsTC;
-    const int c0 = (blockIdx.x % ntx) * kHsTC, r0 = (blockIdx.x / ntx) * kHsTR;
+    const Strip t(P.H, RW);
     const float beta = kFuse ? scal[1] : 0.0f;
-    auto pg = [&](std::int64_t k) { return kFuse ? zz[k] + beta * p_src[k] : p_src[k]; };
-    hs_stage_tile(sx, nr, nc, r0, c0, pg);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double pap_d = 0.0;
-#pragma unroll 1
-    for (int qr = 0; qr < 4; ++qr)
-    {
-        const int lr = 1 + w * 4 + qr, r = r0 + lr - 1;
-        if (r >= nr) break;  // warp-uniform
-        const std::int64_t rb = static_cast<std::int64_t>(r) * nc;
+    float pv[RW + 2], zv[RW + 2];
+    float4 av[RW];
+    unsigned kd[RW];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < RW + 2; ++k)
+    {
+        const int row = t.row(k);
+        const bool in = row >= 0;
+        const std::int64_t i = static_cast<std::int64_t>(row) * nc + t.c;
+        pv[k] = in ? p_src[i] : 0.0f;
+        zv[k] = (kFuse && in) ? zz[i] : 0.0f;
+        if (k >= 1 && k <= RW)
         {
-            const int lc = 1 + 32 * k + lane, c = c0 + lc - 1;
-            float pap = 0.0f;
-            if (c < nc)
-            {
-                const std::int64_t i = rb + c;
-                if (kFuse) p_dst[i] = sx[lr][lc];
-                const std::uint8_t kd = dof[i];
-                const float v = hs_op_cell(P, inv_dt, DA, mask, dof, alpha, sx, lr, lc, r, c, i, kd, pg);
-                Ap[i] = v;
-                if (kd) pap = sx[lr][lc] * v;
-            }
-            pap = warp_sum_f(pap);
-            if (lane == 0) pap_d += static_cast<double>(pap);
+            const bool mine = t.own && t.r0 - 1 + k < nr;
+            kd[k - 1] = mine ? dof[i] : 0u;
+            av[k - 1] = mine ? alpha[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-    block_store_d(pap_d, part + blockIdx.x);
+    if (kFuse)
+    {
+#pragma unroll
+        for (int k = 0; k < RW + 2; ++k) pv[k] = zv[k] + beta * pv[k];
+    }
+    Sum2 v[1];
+#pragma unroll
+    for (int k = 1; k <= RW; ++k)
+    {
+        const float pe = __shfl_down_sync(0xffffffffu, pv[k], 1), pw = __shfl_up_sync(0xffffffffu, pv[k], 1);
+        const int row = t.r0 - 1 + k;
+        if (!t.own || row >= nr) continue;
+        const std::int64_t i = static_cast<std::int64_t>(row) * nc + t.c;
+        const float pi = pv[k];
+        const float4 a = av[k - 1];
+        const unsigned cl = kd[k - 1];
+        float s = 0.0f;
+        s += (cl & 4u) ? a.x * (pi - pv[k - 1]) : 0.0f;
+        s += (cl & 8u) ? a.y * (pi - pe) : 0.0f;
+        s += (cl & 16u) ? a.z * (pi - pv[k + 1]) : 0.0f;
+        s += (cl & 32u) ? a.w * (pi - pw) : 0.0f;
+        const float o = cl ? inv_dt * pi + DA * s : 0.0f;
+        if (kFuse) p_dst[i] = pi;
+        Ap[i] = o;
+        if (cl) v[0].add(pi * o);
+    }
+    const unsigned nblk = gridDim.x;
+    block_partials<1>(v, part, nblk);
+    if (!last_block(&L->arrived, nblk)) return;
+    double s[1];
+    total_partials<1>(part, nblk, s);
+    if (threadIdx.x == 0)
+    {
+        *pap_out = s[0];
+        scal[0] = s[0] > 0.0 ? static_cast<float>(*rz / s[0]) : 0.0f;
+    }
 }
 
 // The smoothing step of the learned preconditioner over one tile per block:
@@ -689,44 +967,70 @@ __global__ void __launch_bounds__(256) hsf_smooth_t(HsN P, float inv_dt, float D
 }
 
 // Jacobi-PCG update with alpha = scal[0]: x += alpha p; r -= alpha Ap;
-// zz = D^-1 r; partials part[blk] = r.z, part[G + blk] = r.r (G blocks,
-// grid-stride over 32-cell warp rows).
-__global__ void __launch_bounds__(256) hs_update_g(std::int64_t n, const float* __restrict__ scal,
+// zz = D^-1 r; r.z and r.r into out[0], out[1] (FP32 over four cells, two
+// words beyond), from which the last block forms beta = r.z / *rz (scal[1]) and
+// tests convergence every fourth iteration. Four cells a thread and access.
+__global__ void __launch_bounds__(256) hs_update_g(std::int64_t n, float* __restrict__ scal,
                                                   const float* __restrict__ inv_diag, const float* __restrict__ p,
                                                   const float* __restrict__ Ap, float* __restrict__ x,
                                                   float* __restrict__ r, float* __restrict__ zz,
-                                                  double* __restrict__ part)
+                                                  double* __restrict__ part, HsnLoop* __restrict__ L,
+                                                  const double* __restrict__ rz, double* __restrict__ out, double bnorm,
+                                                  double rel_tol, int max_iter)
 {
     LSDTT_COUNT();
+    if (L->done) return;
     const float alpha = scal[0];
-    const int lane = threadIdx.x & 31;
-    double rz_d = 0.0, rr_d = 0.0;
-    const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
-    for (std::int64_t b = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); b < n;
-         b += stride)
+    Sum2 v[2];
+    const std::int64_t t0 = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x, n4 = n >> 2;
+    for (std::int64_t q = t0; q < n4; q += stride)
     {
-        const std::int64_t i = b + lane;
-        float rz = 0.0f, rr = 0.0f;
-        if (i < n)
+        const float4 pv = reinterpret_cast<const float4*>(p)[q], av = reinterpret_cast<const float4*>(Ap)[q];
+        const float4 dv = reinterpret_cast<const float4*>(inv_diag)[q];
+        float4 xv = reinterpret_cast<float4*>(x)[q], rv = reinterpret_cast<float4*>(r)[q];
+        xv.x += alpha * pv.x;
+        xv.y += alpha * pv.y;
+        xv.z += alpha * pv.z;
+        xv.w += alpha * pv.w;
+        rv.x -= alpha * av.x;
+        rv.y -= alpha * av.y;
+        rv.z -= alpha * av.z;
+        rv.w -= alpha * av.w;
+        const float4 zv = make_float4(rv.x * dv.x, rv.y * dv.y, rv.z * dv.z, rv.w * dv.w);
+        reinterpret_cast<float4*>(x)[q] = xv;
+        reinterpret_cast<float4*>(r)[q] = rv;
+        reinterpret_cast<float4*>(zz)[q] = zv;
+        v[0].add((rv.x * zv.x + rv.y * zv.y) + (rv.z * zv.z + rv.w * zv.w));
+        v[1].add((rv.x * rv.x + rv.y * rv.y) + (rv.z * rv.z + rv.w * rv.w));
+    }
+    if (t0 < (n & 3))
+    {
+        const std::int64_t i = 4 * n4 + t0;
+        x[i] += alpha * p[i];
+        const float ri = r[i] - alpha * Ap[i], zi = ri * inv_diag[i];
+        r[i] = ri;
+        zz[i] = zi;
+        v[0].add(ri * zi);
+        v[1].add(ri * ri);
+    }
+    const unsigned nblk = gridDim.x;
+    block_partials<2>(v, part, nblk);
+    if (!last_block(&L->arrived, nblk)) return;
+    double t[2];
+    total_partials<2>(part, nblk, t);
+    if (threadIdx.x == 0)
+    {
+        out[0] = t[0];
+        out[1] = t[1];
+        scal[1] = *rz > 0.0 ? static_cast<float>(t[0] / *rz) : 0.0f;
+        const int it = ++L->iters;
+        if (it % 4 == 0 || it >= max_iter)
         {
-            x[i] += alpha * p[i];
-            const float ri = r[i] - alpha * Ap[i];
-            r[i] = ri;
-            const float zi = ri * inv_diag[i];
-            zz[i] = zi;
-            rz = ri * zi;
-            rr = ri * ri;
-        }
-        rz = warp_sum_f(rz);
-        rr = warp_sum_f(rr);
-        if (lane == 0)
-        {
-            rz_d += static_cast<double>(rz);
-            rr_d += static_cast<double>(rr);
+            L->rel = sqrt(t[1]) / bnorm;
+            if (L->rel <= rel_tol) L->done = 1;
         }
     }
-    block_store_d(rz_d, part + blockIdx.x);
-    block_store_d(rr_d, part + gridDim.x + blockIdx.x);
 }
 
 // Flexible-PCG update with alpha = scal[0]: x += alpha p; r_old = r;
@@ -924,6 +1228,7 @@ struct HsnBuf
     float* p2;     // the other direction buffer of the fused apply
     double* part;  // block partials: 4 x tiles, then 2 x kHsUpdBlocks
     float* scal;   // [0] alpha, [1] beta of the current iteration
+    HsnLoop* loop; // the loop's state, in the same 256 bytes
     double* hacc;
 };
 
@@ -945,6 +1250,7 @@ void hsn_pcg_carve(HsnBuf& B, int nr, int nc, Carve carve)
     B.part = reinterpret_cast<double*>(
         carve(sizeof(double) * (4 * static_cast<std::size_t>(hs_tiles(nr, nc)) + 2 * kHsUpdBlocks)));
     B.scal = reinterpret_cast<float*>(carve(256));
+    B.loop = reinterpret_cast<HsnLoop*>(B.scal + 16);
 }
 
 // Statistics of the linear solves of one hillslope call.
@@ -986,14 +1292,27 @@ cudaError_t jacobi_loop(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::
     float* pbuf[2] = {B.p, B.p2};
     double* part_ap = B.part;
     double* part_up = B.part + 4 * static_cast<std::size_t>(tiles);
-    int it = 0;
+    const bool tall = strip_long(P.H.nr, P.H.nc);
+    const unsigned nt = strip_blocks(P.H.nr, P.H.nc, tall ? 16 : 8);
+    const unsigned ub = static_cast<unsigned>(std::min<std::int64_t>(kHsUpdBlocks, (n + 1023) / 1024));
+    cudaMemsetAsync(B.loop, 0, sizeof(HsnLoop), st);
+    auto apply = [&](const float* src, float* dst, const double* rz, double* pap, bool fuse) {
+#define LSDTT_APPLY(F, TR)                                                                                            \
+    hsn_apply_t<F, TR><<<nt, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal, B.zz, src, dst, B.Ap, part_ap, \
+                                           B.loop, rz, pap)
+        if (tall && fuse) LSDTT_APPLY(true, 16);
+        else if (tall) LSDTT_APPLY(false, 16);
+        else if (fuse) LSDTT_APPLY(true, 8);
+        else LSDTT_APPLY(false, 8);
+#undef LSDTT_APPLY
+    };
+    int it = 0, step = 4;
     std::size_t next_snap = 0;
-    const int kCheck = 4;
-    bool done = false;
+    HsnLoop H{};
     cudaError_t e = cudaSuccess;
-    while (!done && it < max_iter)
+    while (it < max_iter)
     {
-        const int batch = std::min(kCheck, max_iter - it);
+        const int batch = std::min(step, max_iter - it);
         for (int k = 0; k < batch; ++k, ++it)
         {
             double* cur = slots + kSlot * it;
@@ -1001,22 +1320,10 @@ cudaError_t jacobi_loop(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::
             // the direction p = z + beta p of the previous iteration is
             // formed inside the apply (the first iteration's p is given)
             float* p = pbuf[it & 1];
-            if (it == 0)
-                LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
-                            (hsn_apply_t<false><<<tiles, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal,
-                                                                       B.zz, p, p, B.Ap, part_ap)));
-            else
-                LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
-                            (hsn_apply_t<true><<<tiles, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal,
-                                                                      B.zz, pbuf[(it - 1) & 1], p, B.Ap, part_ap)));
-            // p.Ap, alpha = rz_prev / p.Ap
-            hs_reduce<<<1, 512, 0, st>>>(HsRed{{part_ap, nullptr, nullptr, nullptr}, {tiles, 0, 0, 0},
-                                               {cur, nullptr, nullptr, nullptr}, rz_prev, cur, B.scal});
-            hs_update_g<<<kHsUpdBlocks, 256, 0, st>>>(n, B.scal, B.invd, p, B.Ap, B.x, B.r, B.zz, part_up);
-            // r.z, r.r, beta = r.z / rz_prev
-            hs_reduce<<<1, 512, 0, st>>>(HsRed{{nullptr, part_up, part_up + kHsUpdBlocks, nullptr},
-                                               {0, kHsUpdBlocks, kHsUpdBlocks, 0},
-                                               {nullptr, cur + 1, cur + 2, nullptr}, cur + 1, rz_prev, B.scal + 1});
+            LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
+                        (apply(it == 0 ? p : pbuf[(it - 1) & 1], p, rz_prev, cur, it > 0)));
+            hs_update_g<<<ub, 256, 0, st>>>(n, B.scal, B.invd, p, B.Ap, B.x, B.r, B.zz, part_up, B.loop, rz_prev,
+                                            cur + 1, bnorm, check ? rel_tol : -1.0, max_iter);
             while (snap_at && next_snap < snap_at->size() && (*snap_at)[next_snap] == it)
             {
                 cudaMemcpyAsync(x_snap + next_snap * n, B.x, sizeof(float) * n, cudaMemcpyDeviceToDevice, st);
@@ -1025,13 +1332,15 @@ cudaError_t jacobi_loop(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::
             }
         }
         if (!check) continue;
-        cudaMemcpyAsync(B.hacc, slots + kSlot * (it - 1), sizeof(double) * 3, cudaMemcpyDeviceToHost, st);
+        // (a batch launched past convergence returns at once)
+        cudaMemcpyAsync(&H, B.loop, sizeof(H), cudaMemcpyDeviceToHost, st);
         e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return e;
-        *rel = std::sqrt(B.hacc[2]) / bnorm;
-        done = *rel <= rel_tol;
+        *rel = H.rel;
+        if (H.done) break;
+        step = std::min(16, step + 4);
     }
-    *iters = it;
+    *iters = check ? H.iters : it;
     return cudaGetLastError();
 }
 
@@ -1092,6 +1401,7 @@ cudaError_t hsn_pcg(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::int6
     double* part_ap = B.part;
     double* part_rz = B.part + tiles;
     double* part_roz = B.part + 2 * static_cast<std::size_t>(tiles);
+    const unsigned nt = strip_blocks(H, W, 8);
     double* part_rr = B.part + 4 * static_cast<std::size_t>(tiles);
     // z = y + D^-1 (r - A y), y = the network applied to q = D^-1 r (in zz),
     // masked to the DOFs; partials of r.z and z.(r - r_old)
@@ -1103,6 +1413,7 @@ cudaError_t hsn_pcg(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::int6
                                             part_rz, part_roz);
         return pe;
     };
+    cudaMemsetAsync(B.loop, 0, sizeof(HsnLoop), st);
     cudaMemcpyAsync(B.ro, B.r, sizeof(float) * n, cudaMemcpyDeviceToDevice, st);
     hsf_input<<<nb, 256, 0, st>>>(n, B.invd, B.r, B.zz);
     e = precondition();
@@ -1123,17 +1434,17 @@ cudaError_t hsn_pcg(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::int6
             const double* rz_prev = (it == 0) ? acc + 9 : slots + kSlot * (it - 1) + 1;
             // p = z + beta p of the previous iteration inside the apply
             float* p = pbuf[it & 1];
+            // (with p.Ap and alpha = rz_prev / p.Ap)
             if (it == 0)
                 LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
-                            (hsn_apply_t<false><<<tiles, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal,
-                                                                       B.zz, p, p, B.Ap, part_ap)));
+                            (hsn_apply_t<false, 8><<<nt, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha,
+                                                                              B.scal, B.zz, p, p, B.Ap, part_ap, B.loop,
+                                                                              rz_prev, cur)));
             else
                 LSDTT_TIMED("hillslope_apply", 8.0 * static_cast<double>(n), st,
-                            (hsn_apply_t<true><<<tiles, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal,
-                                                                      B.zz, pbuf[(it - 1) & 1], p, B.Ap, part_ap)));
-            // p.Ap, alpha = rz_prev / p.Ap
-            hs_reduce<<<1, 512, 0, st>>>(HsRed{{part_ap, nullptr, nullptr, nullptr}, {tiles, 0, 0, 0},
-                                               {cur, nullptr, nullptr, nullptr}, rz_prev, cur, B.scal});
+                            (hsn_apply_t<true, 8><<<nt, 256, 0, st>>>(P, inv_dt, DA, mask, B.dof, B.alpha, B.scal,
+                                                                             B.zz, pbuf[(it - 1) & 1], p, B.Ap, part_ap,
+                                                                             B.loop, rz_prev, cur)));
             hsf_update_g<<<kHsUpdBlocks, 256, 0, st>>>(n, B.scal, B.invd, p, B.Ap, B.x, B.r, B.ro, B.zz, part_rr);
             e = precondition();
             // r.z, r.r, z.(r - r_old); beta = z.(r - r_old) / rz_prev (Polak-Ribiere)
@@ -1268,10 +1579,8 @@ int hillslope_implicit_impl(const std::string& who, const lsdtt_gpu_grid* grid, 
     double* acc_it = reinterpret_cast<double*>(carve(sizeof(double) * solve_acc_doubles(kPcg)));
     hsn_pcg_carve(B, P.H.nr, P.H.nc, carve);
     SolveStats S;
-    // DOF mask via the linear set-up kernel (it only needs mask, channels, edges).
     {
-        double* junk = B.F;
-        hs_setup<<<nb, 256, 0, st>>>(P.H, mask_dev, is_channel_dev, z_dev, z_dev, B.dof, B.invd, B.b, junk);
+        hs_dofs<<<nb, 256, 0, st>>>(P.H, mask_dev, is_channel_dev, B.dof);
     }
     hsn_to_double<<<nb, 256, 0, st>>>(n, z_dev, B.z);
     cudaMemcpyAsync(B.zn, B.z, 8 * n, cudaMemcpyDeviceToDevice, st);
@@ -1486,7 +1795,7 @@ extern "C" int lsdtt_gpu_hillslope_capture_pairs(const lsdtt_gpu_grid* grid, con
     B.acc = reinterpret_cast<double*>(carve(sizeof(double) * 8));
     double* acc = reinterpret_cast<double*>(carve(sizeof(double) * solve_acc_doubles(kPcg)));
     hsn_pcg_carve(B, P.H.nr, P.H.nc, carve);
-    hs_setup<<<nb, 256, 0, st>>>(P.H, mask_dev, is_channel_dev, z_dev, z_dev, B.dof, B.invd, B.b, B.F);
+    hs_dofs<<<nb, 256, 0, st>>>(P.H, mask_dev, is_channel_dev, B.dof);
     hsn_to_double<<<nb, 256, 0, st>>>(n, z_dev, B.z);
     double ev[3];
     e = hsn_evaluate(P, mask_dev, B, B.z, n, st, ev);
