@@ -44,6 +44,60 @@ __device__ __forceinline__ double sp_kam(const SpParams& P, double area_d, float
     return __dmul_rn(static_cast<double>(Ki), pow(area, static_cast<double>(P.m)));
 }
 
+// ---- the update in two FP32 words -------------------------------------------
+// The reference solves a node in FP64 and rounds to float once per step. This
+// part's FP64 pipe takes 16 cycles an instruction and warp, and a node is 13
+// (n = 1) or several hundred of them (division and square root are sequences),
+// so the sweeps were bound by it. The same values are formed here in pairs of
+// FP32 words (error-free sums and products), right to about 2^-44 of their
+// terms where the FP64 ones are right to 2^-51. Where both ends of that
+// interval lead to the same float (and to the same answer of the loop's test),
+// it is the float that the FP64 expression gives; where they do not, the FP64
+// expression is evaluated. So the bits are the reference's, and FP64 is left
+// for about one node in 10^4.
+
+// float((zo + zr spf) / (1 + spf)) = zr + (zo - zr) w for w = 1 / (1 + spf)
+// = wh + wl, zr < zo; false where FP64 has to decide.
+__device__ __forceinline__ bool sp_linear_pair(float wh, float wl, float zo, float zr, float& zn)
+{
+    const float d = zo - zr, bb = d - zo, dl = (zo - (d - bb)) - (zr + bb);
+    const float ph = d * wh, pl = fmaf(d, wh, -ph) + fmaf(d, wl, dl * wh);
+    const float s = zr + ph, t = s - zr, lo = ((zr - (s - t)) + (ph - t)) + pl;
+    const float size = fabsf(zr) + fabsf(zo), err = size * 5.6843419e-14f;  // 2^-44
+    const float up = s + (lo + err), dn = s + (lo - err);
+    zn = up;
+    return up == dn && size > 1e-20f && size < 1e30f;
+}
+
+// A Newton step of the n = 1.5 or n = 2 update: zn - float(eps) for eps = fz /
+// fdz, fz = (zn - zo) + kdt s^n, fdz = 1 + kdt ndx s^(n-1) (kdt = kh + kl, kdt
+// ndx = gh + gl), and whether |eps| > tol; false where FP64 has to decide.
+__device__ __forceinline__ bool sp_newton_pair(bool square, float s, float kh, float kl, float gh, float gl, float dz,
+                                               float tol, float zn, float& z_next, bool& again)
+{
+    // p = s^n and r = s^(n-1)
+    float rh = s, rl = 0.0f;
+    if (!square)
+    {
+        rh = __fsqrt_rn(s);
+        rl = 0.5f * fmaf(-rh, rh, s) * __frcp_rn(rh);
+    }
+    const float ph = s * rh, pl = fmaf(s, rh, -ph) + s * rl;
+    const float th = kh * ph, tl = fmaf(kh, ph, -th) + fmaf(kh, pl, kl * ph);
+    const float fh = dz + th, a = fh - dz, fl = ((dz - (fh - a)) + (th - a)) + tl;
+    const float uh = gh * rh, ul = fmaf(gh, rh, -uh) + fmaf(gh, rl, gl * rh);
+    const float qh = 1.0f + uh, b = qh - 1.0f, ql = ((1.0f - (qh - b)) + (uh - b)) + ul;
+    const float inv = __frcp_rn(qh), e0 = fh * inv;
+    const float e1 = (fmaf(-e0, qh, fh) + fmaf(-e0, ql, fl)) * inv;
+    const float err = (fabsf(dz) + th) * inv * 2.2737368e-13f;  // 2^-42
+    const float up = e0 + (e1 + err), dn = e0 + (e1 - err);
+    z_next = zn - up;
+    const float au = fabsf(up), ad = fabsf(dn);
+    again = au > tol;
+    const bool clear = fminf(au, ad) > tol * 1.000001f || fmaxf(au, ad) < tol * 0.999999f;
+    return z_next == zn - dn && clear && th < 1e30f && uh < 1e30f && err > 1e-36f;
+}
+
 // The implicit update of one node (stream_power_cpu.cpp:263-318): its new
 // elevation from its own old elevation zo, its receiver's final elevation
 // zr, kam = sp_kam(...) and the step length to the receiver. Returns zo when
@@ -60,6 +114,17 @@ __device__ __forceinline__ float sp_solve_tol(const SpParams& P, bool diagonal, 
     float zn = zo;
     if (P.n_is_one)
     {
+        // w = 1 / (1 + spf) from spf in two words
+        const float q = __fdiv_rn(P.dt, dx_eff);
+        const float kh = static_cast<float>(kam), kl = static_cast<float>(kam - static_cast<double>(kh));
+        const float sh = kh * q, sl = fmaf(kh, q, -sh) + kl * q;
+        const float dh = 1.0f + sh, b = dh - 1.0f, dl = ((1.0f - (dh - b)) + (sh - b)) + sl;
+        const float wh = __frcp_rn(dh), wl = (fmaf(-wh, dh, 1.0f) - wh * dl) * wh;
+        if (sh < 1e15f && sh > 1e-30f && sp_linear_pair(wh, wl, zo, zr, zn))
+        {
+            if (__fsub_rn(zn, zo) > static_cast<float>(tol) || isnan(zn)) zn = zo;
+            return zn;
+        }
         const double spf = __dmul_rn(kam, static_cast<double>(__fdiv_rn(P.dt, dx_eff)));
         const double num = __dadd_rn(static_cast<double>(zo), __dmul_rn(static_cast<double>(zr), spf));
         zn = static_cast<float>(__ddiv_rn(num, __dadd_rn(1.0, spf)));
@@ -67,17 +132,33 @@ __device__ __forceinline__ float sp_solve_tol(const SpParams& P, bool diagonal, 
     }
     else
     {
-        double eps = tol + 1.0;
+        double eps = 0.0;
         int it = 0;
         const double nd = static_cast<double>(P.n);
         const double kdt = __dmul_rn(kam, static_cast<double>(P.dt));
-        const double ndx = static_cast<double>(__fdiv_rn(P.n, dx_eff));
-        do
+        const float ndxf = __fdiv_rn(P.n, dx_eff);
+        const double ndx = static_cast<double>(ndxf);
+        const bool square = P.n == 2.0f;
+        const float kh = static_cast<float>(kdt), kl = static_cast<float>(kdt - static_cast<double>(kh));
+        const float gh = kh * ndxf, gl = fmaf(kh, ndxf, -gh) + kl * ndxf, tolf = static_cast<float>(tol);
+        const bool pair = (square || P.n == 1.5f) && kh > 1e-25f && gh > 1e-25f;
+        for (;;)
         {
-            const double slope = static_cast<double>(__fdiv_rn(__fsub_rn(zn, zr), dx_eff));
-            if (slope <= 0.0) eps = 0.0;
+            const float sf = __fdiv_rn(__fsub_rn(zn, zr), dx_eff);
+            if (sf <= 0.0f) eps = 0.0;
             else
             {
+                float next;
+                bool again;
+                if (pair && it < 100 && sf > 1e-10f &&
+                    sp_newton_pair(square, sf, kh, kl, gh, gl, __fsub_rn(zn, zo), tolf, zn, next, again))
+                {
+                    zn = next;
+                    ++it;
+                    if (again) continue;
+                    break;
+                }
+                const double slope = static_cast<double>(sf);
                 const double fz = __dadd_rn(static_cast<double>(__fsub_rn(zn, zo)), __dmul_rn(kdt, sp_pow(slope, nd)));
                 const double fdz =
                     __dadd_rn(1.0, __dmul_rn(__dmul_rn(kdt, ndx), sp_pow(slope, __dsub_rn(nd, 1.0))));
@@ -86,7 +167,8 @@ __device__ __forceinline__ float sp_solve_tol(const SpParams& P, bool diagonal, 
             zn = __fsub_rn(zn, static_cast<float>(eps));
             ++it;
             if (it > 100) eps = tol / 2.0;
-        } while (fabs(eps) > tol);
+            if (!(fabs(eps) > tol)) break;
+        }
         if (__fsub_rn(zn, zo) > static_cast<float>(tol) || isnan(zn)) zn = zo;
         if (zn < zr) zn = __fadd_rn(zr, __fmul_rn(P.slope_clamp, dx_eff));
     }
