@@ -242,7 +242,7 @@ std::size_t exact_single_bytes(std::int64_t n)
 // bytes. F holds the epsilon relaxation on entry. Allocates nothing.
 cudaError_t exact_fill_single_in(int nr, int nc, bool per_ns, bool per_ew, float L, float Ld, float eps, float nodata,
                                  const float* z, const std::uint8_t* kind, const float* F0, float* F, char* buf,
-                                 cudaStream_t st, unsigned* failure)
+                                 cudaStream_t st, unsigned* failure, const ExSide* side = nullptr)
 {
     *failure = 0;
     const std::int64_t n = static_cast<std::int64_t>(nr) * nc;
@@ -279,7 +279,7 @@ cudaError_t exact_fill_single_in(int nr, int nc, bool per_ns, bool per_ew, float
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = ex_run(mem, blk, N, 1, 0, z, kind, F0, F, B, ws, std::max(sms, 1), st);
+    if (e == cudaSuccess) e = ex_run(mem, blk, N, 1, 0, z, kind, F0, F, B, ws, std::max(sms, 1), st, false, -1, side);
     unsigned hu[6] = {0, 0, 0, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(hu, B.u, sizeof(hu), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -296,7 +296,21 @@ cudaError_t exact_fill_single(int nr, int nc, bool per_ns, bool per_ew, float L,
     char* buf = nullptr;
     cudaError_t e = cudaMallocAsync(&buf, exact_single_bytes(static_cast<std::int64_t>(nr) * nc), st);
     if (e != cudaSuccess) return e;
-    e = exact_fill_single_in(nr, nc, per_ns, per_ew, L, Ld, eps, nodata, z, kind, F0, F, buf, st, failure);
+    // (profiled launches stay on one stream, one after another)
+    ExSide side;
+    cudaError_t se = profiling_enabled() ? cudaErrorNotSupported
+                                         : cudaStreamCreateWithFlags(&side.st, cudaStreamNonBlocking);
+    if (se == cudaSuccess) se = cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming);
+    if (se == cudaSuccess) se = cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming);
+    e = exact_fill_single_in(nr, nc, per_ns, per_ew, L, Ld, eps, nodata, z, kind, F0, F, buf, st, failure,
+                             se == cudaSuccess ? &side : nullptr);
+    if (side.fork) cudaEventDestroy(side.fork);
+    if (side.join) cudaEventDestroy(side.join);
+    if (side.st)
+    {
+        if (e != cudaSuccess) cudaStreamSynchronize(side.st);  // nothing of it outlives the buffers
+        cudaStreamDestroy(side.st);
+    }
     cudaFreeAsync(buf, st);
     return e;
 }

@@ -67,7 +67,7 @@ struct ExBuffers
     std::int64_t* nsorted;  // [M]
     int *ncut, *cut_base;   // [M], [M + 1]
     unsigned* u;            // [0] total cuts, [1] nwl, [2] work, [3] nwl2, [4] work2, [5] error,
-                            // [6] nwl3, [7] work3, [8] pour keys
+                            // [6] nwl3, [7] work3, [8] pour keys, [9] chains done
     unsigned long long* pool_used;
 };
 
@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(32) ex_windows(const ExMember* __restrict__ me
                                                  const std::uint8_t* __restrict__ kind, const float* __restrict__ F0,
                                                  ExBuffers B, const std::int32_t* __restrict__ wl,
                                                  const unsigned* __restrict__ nwl, unsigned* __restrict__ work,
-                                                 unsigned long long pool_cap, unsigned long long pop_limit)
+                                                 unsigned long long pool_cap, unsigned long long pop_limit,
+                                                 unsigned min_windows, const unsigned* __restrict__ chain_done)
 {
     LSDTT_COUNT();
     extern __shared__ __align__(16) unsigned char ex_smem[];
@@ -350,8 +351,10 @@ __global__ void __launch_bounds__(32) ex_windows(const ExMember* __restrict__ me
     s.ocap = OC;
     const int lane = threadIdx.x & 31;
     const unsigned total = *nwl;
+    if (total < min_windows) return;  // (they stay marked as they are)
     for (;;)
     {
+        if (chain_done && *reinterpret_cast<const volatile unsigned*>(chain_done)) break;
         unsigned t = 0;
         if (lane == 0) t = atomicAdd(work, 1u);
         t = __shfl_sync(0xffffffffu, t, 0);
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(32) ex_windows(const ExMember* __restrict__ me
         const int g = wl[t];
         const int m = B.cut_member[g];
         const WinGrid G = ex_member_grid(mem[m], m, z, kind, F0, B);
-        WinResult r = win_replay(G, g - B.cut_base[m], s, pop_limit);
+        WinResult r = win_replay(G, g - B.cut_base[m], s, pop_limit, chain_done);
         unsigned long long base = 0;
         if (r.status == kWinOk && r.nout)
         {
@@ -373,12 +376,14 @@ __global__ void __launch_bounds__(32) ex_windows(const ExMember* __restrict__ me
                     B.pool_v[base + k] = s.ov[k];
                 }
         }
+        __syncwarp();
         if (lane == 0)
         {
             B.next[g] = r.next;
-            B.status[g] = static_cast<std::uint8_t>(r.status);
             B.off[g] = static_cast<std::uint32_t>(base);
             B.cnt[g] = r.nout;
+            __threadfence();  // a chain that runs beside this reads the status first
+            *reinterpret_cast<volatile std::uint8_t*>(&B.status[g]) = static_cast<std::uint8_t>(r.status);
         }
         __syncwarp();
     }
@@ -453,18 +458,58 @@ __global__ void __launch_bounds__(kSwThreads) ex_chain(const ExMember* __restric
     big.hk = B.ghk + M.base;
     big.hcap = static_cast<std::uint32_t>(static_cast<std::int64_t>(M.nr) * M.nc);
     __shared__ std::uint32_t s_ctr;
-    __shared__ int s_nx, s_fail;
+    __shared__ int s_nx, s_fail, s_replay;
     if (tid == 0)
     {
         s_ctr = B.sw_ctr[m];
         s_fail = 0;
     }
     __syncthreads();
+    // The chain is followed through blocks of kSwThreads cuts in shared memory
+    // (next window, or -1 where no size held the window): a step there is a
+    // shared load, in global memory it was two dependent ones and a barrier.
+    int* nxt = reinterpret_cast<int*>(ex_csmem);
     int w = 0;
     while (w < G.ncut)
     {
+        const int at = w + tid;
+        int y0 = -1;
+        if (at < G.ncut && *reinterpret_cast<volatile std::uint8_t*>(&B.status[cb + at]) == kWinOk)
+        {
+            __threadfence();
+            y0 = __ldcg(B.next + cb + at);
+        }
+        nxt[tid] = y0;
+        __syncthreads();
+        if (tid == 0)
+        {
+            int x = w;
+            while (x < G.ncut && x - w < kSwThreads)
+            {
+                const int y = nxt[x - w];
+                if (y < 0) break;
+                B.chain[cb + x] = 1;
+                if (y <= x)  // a window always ends above its start
+                {
+                    s_fail = 2;
+                    break;
+                }
+                x = y;
+            }
+            s_nx = x;
+            s_replay = x < G.ncut && x - w < kSwThreads ? 1 : 0;
+        }
+        __syncthreads();
+        if (s_fail)
+        {
+            if (tid == 0) atomicExch(&B.u[5], 2u);
+            return;
+        }
+        w = s_nx;
+        const bool replay = s_replay != 0;
+        __syncthreads();
+        if (!replay) continue;
         int nx;
-        if (B.status[cb + w] != kWinOk)
         {
             int sn = G.ncut;
             const int rs = win_sweep_replay(G, w, sb, F + M.base, &s_ctr, sh, &sn);
@@ -499,11 +544,6 @@ __global__ void __launch_bounds__(kSwThreads) ex_chain(const ExMember* __restric
             }
             if (tid == 0) B.chain[cb + w] = 2;
         }
-        else
-        {
-            nx = B.next[cb + w];
-            if (tid == 0) B.chain[cb + w] = 1;
-        }
         __syncthreads();
         if (nx <= w)  // a window always ends above its start
         {
@@ -512,7 +552,11 @@ __global__ void __launch_bounds__(kSwThreads) ex_chain(const ExMember* __restric
         }
         w = nx;
     }
-    if (tid == 0) B.sw_ctr[m] = s_ctr;
+    if (tid == 0)
+    {
+        B.sw_ctr[m] = s_ctr;
+        atomicAdd(&B.u[9], 1u);  // (read by replays that run beside a single chain)
+    }
 }
 
 // 7. Staged raised cells of the chain windows into F, one warp per window.
@@ -536,12 +580,27 @@ constexpr int kExA_FQ = 128, kExA_DH = 256, kExA_HS = 1024, kExA_OC = 256;
 // (windows past the small size are heap-bound: their FIFO stays short)
 constexpr int kExM_FQ = 128, kExM_DH = 1024, kExM_HS = 4096, kExM_OC = 512;
 constexpr int kExB_FQ = 128, kExB_DH = 4096, kExB_HS = 8192, kExB_OC = 1024;
+// Fewer overflowing windows than this are left to the chains where the larger
+// sizes cannot run beside them: a one-warp replay takes about 1.5 us a pop and
+// its longest window is its time, a block sweep 0.06-0.5 us a pop but one
+// window after another. (12, 24, 48, 160: a 700 x 600 pitted fractal 32.5,
+// 32.4, 36.7, 49.1 ms; always replayed first, a 512 x 512 noise tilt takes
+// 27.7 ms and not 22.3.)
+constexpr unsigned kExMinWindows = 20;
 constexpr std::size_t kExSmemA = 8 * kExA_FQ + 8 * (kExA_DH + 2) + 4 * kExA_HS + 8 * kExA_OC;
 constexpr std::size_t kExSmemM = 8 * kExM_FQ + 8 * (kExM_DH + 2) + 4 * kExM_HS + 8 * kExM_OC;
 constexpr std::size_t kExSmemB = 8 * kExB_FQ + 8 * (kExB_DH + 2) + 4 * kExB_HS + 8 * kExB_OC;
 constexpr int kExC_FQ = 2048, kExC_DH = 16384;
 constexpr std::size_t kExSmemC =
     (8 * kExC_FQ + 8 * (kExC_DH + 2)) > sizeof(SweepShared) ? (8 * kExC_FQ + 8 * (kExC_DH + 2)) : sizeof(SweepShared);
+
+// A second stream (and its fork and join events) of a single-grid fill: the
+// larger replay sizes run on it beside the chain.
+struct ExSide
+{
+    cudaStream_t st = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
 
 // Opt the larger replay sizes into their shared memory (current device).
 inline cudaError_t ex_setup()
@@ -569,7 +628,8 @@ inline cudaError_t ex_setup()
 // the members whose fill is on (their chains are the ones that work).
 inline cudaError_t ex_run(const ExMember* mem, const std::uint16_t* blk_member, std::int64_t N, int M, int mbits,
                           const float* z, const std::uint8_t* kind, const float* F0, float* F, const ExBuffers& B,
-                          Scratch& ws, int sms, cudaStream_t st, bool ens = false, int n_on = -1)
+                          Scratch& ws, int sms, cudaStream_t st, bool ens = false, int n_on = -1,
+                          const ExSide* side = nullptr)
 {
     if (n_on < 0) n_on = M;
     static const char* const kNames[2][9] = {
@@ -646,25 +706,44 @@ inline cudaError_t ex_run(const ExMember* mem, const std::uint16_t* blk_member, 
     // small size could not hold -- only those on a chain, where the larger
     // sizes replay every such candidate one pop at a time -- and the step
     // is faster without them (256 members: 358 ms a step with them, 234 ms
-    // without; one 2048 x 2048 grid: 498 ms with them, 779 ms without)
+    // without; one 2048 x 2048 grid: 498 ms with them, 779 ms without).
+    // A single grid's chain is one block: with `side` the larger sizes run
+    // beside it on the other SMs. The chain takes what they have finished when
+    // it gets there and replays the rest itself, and they stop when it is
+    // done; whichever replays a window, its raised cells are the same.
+    auto larger = [&](cudaStream_t s, unsigned min_windows, const unsigned* done) {
+        LSDTT_TIMED(nm[5], 16.0 * cells, s,
+                    (ex_overflow_list<<<nb, 256, 0, s>>>(N, B.wl, B.u + 1, B.wl2, B.u + 3, B.status),
+                     ex_windows<kExM_FQ, kExM_DH, kExM_HS, kExM_OC><<<sms * 7, 32, kExSmemM, s>>>(
+                         mem, z, kind, F0, B, B.wl2, B.u + 3, B.u + 4, static_cast<unsigned long long>(N),
+                         16ull * kExM_HS, min_windows, done)));
+        LSDTT_TIMED(nm[6], 16.0 * cells, s,
+                    (ex_overflow_list<<<nb, 256, 0, s>>>(N, B.wl2, B.u + 3, B.wl, B.u + 6, B.status),
+                     ex_windows<kExB_FQ, kExB_DH, kExB_HS, kExB_OC><<<sms * 3, 32, kExSmemB, s>>>(
+                         mem, z, kind, F0, B, B.wl, B.u + 6, B.u + 7, static_cast<unsigned long long>(N),
+                         16ull * kExB_HS, min_windows, done)));
+    };
     LSDTT_TIMED(nm[4], 16.0 * cells, st,
                 (ex_windows<kExA_FQ, kExA_DH, kExA_HS, kExA_OC><<<sms * 20, 32, kExSmemA, st>>>(
-                    mem, z, kind, F0, B, B.wl, B.u + 1, B.u + 2, static_cast<unsigned long long>(N), 16ull * kExA_HS)));
-    if (n_on < sms)
+                    mem, z, kind, F0, B, B.wl, B.u + 1, B.u + 2, static_cast<unsigned long long>(N), 16ull * kExA_HS,
+                    0u, nullptr)));
+    if (side && e == cudaSuccess)
     {
-        LSDTT_TIMED(nm[5], 16.0 * cells, st,
-                    (ex_overflow_list<<<nb, 256, 0, st>>>(N, B.wl, B.u + 1, B.wl2, B.u + 3, B.status),
-                     ex_windows<kExM_FQ, kExM_DH, kExM_HS, kExM_OC><<<sms * 7, 32, kExSmemM, st>>>(
-                         mem, z, kind, F0, B, B.wl2, B.u + 3, B.u + 4, static_cast<unsigned long long>(N),
-                         16ull * kExM_HS)));
-        LSDTT_TIMED(nm[6], 16.0 * cells, st,
-                    (ex_overflow_list<<<nb, 256, 0, st>>>(N, B.wl2, B.u + 3, B.wl, B.u + 6, B.status),
-                     ex_windows<kExB_FQ, kExB_DH, kExB_HS, kExB_OC><<<sms * 3, 32, kExSmemB, st>>>(
-                         mem, z, kind, F0, B, B.wl, B.u + 6, B.u + 7, static_cast<unsigned long long>(N),
-                         16ull * kExB_HS)));
+        e = cudaEventRecord(side->fork, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side->st, side->fork, 0);
+        if (e != cudaSuccess) return e;
     }
+    else if (n_on < sms)
+        larger(st, kExMinWindows, nullptr);
     LSDTT_TIMED(nm[7], 16.0 * cells, st,
                 (ex_chain<kExC_FQ, kExC_DH><<<M, kSwThreads, kExSmemC, st>>>(mem, z, kind, F0, F, B)));
+    if (side)
+    {
+        larger(side->st, 0u, B.u + 9);
+        e = cudaEventRecord(side->join, side->st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, side->join, 0);
+        if (e != cudaSuccess) return e;
+    }
     // the staged raised cells: cell 4 + value 4 in, 4 out at most per cell
     LSDTT_TIMED(nm[8], 12.0 * cells, st,
                 (ex_commit<<<static_cast<unsigned>(std::max<std::int64_t>(1, std::min<std::int64_t>(N / 8, sms * 64))),

@@ -1118,6 +1118,29 @@ __device__ bool sw_narrow(const WinGrid& G, const SweepBufs& B, SweepShared& sh,
     return true;
 }
 
+// First k in [lo, n) with a(k) above the searched value (`above`, monotone in
+// k; n if none), by one full warp: 32 probes a step, where one thread's
+// bisection took a dependent load per halving (21 of them at 2 M cells).
+template <class I, class Above>
+__device__ __forceinline__ I sw_search(I lo, I n, const Above& above)
+{
+    const int lane = threadIdx.x & 31;
+    I hi = n;
+    while (hi - lo > 32)
+    {
+        const I step = (hi - lo + 31) / 32;
+        const I k = lo + static_cast<I>(lane) * step;
+        const unsigned b = __ballot_sync(0xffffffffu, k >= hi || above(k));
+        const int f = b ? __ffs(b) - 1 : 32;
+        const I top = lo + static_cast<I>(f) * step;
+        if (f > 0) lo = lo + static_cast<I>(f - 1) * step + 1;
+        hi = f == 0 ? lo : (top < hi ? top : hi);
+    }
+    const I k = lo + lane;
+    const unsigned b = __ballot_sync(0xffffffffu, k >= hi || above(k));
+    return b ? lo + static_cast<I>(__ffs(b) - 1) : hi;
+}
+
 // Block replay of window w (every thread of a kSwThreads block calls it).
 // *ctr is the member's id counter (stamps), advanced here. Returns kWinOk
 // with *next set, or kWinOverflow (a sweep's FIFO or lists above their
@@ -1137,10 +1160,18 @@ __device__ int win_sweep_replay(const WinGrid& G, int w, const SweepBufs& B, flo
     __shared__ float s_Lb[kSwLv];
     __shared__ int s_j;
     __shared__ int s_cnext, s_next, s_stop;
+    __shared__ unsigned long long s_first;
+    __shared__ float s_lz;
+    __shared__ std::uint32_t s_lc;
+    if (tid < 32)
+    {
+        const std::int64_t p =
+            sw_search<std::int64_t>(0, G.nsorted, [&](std::int64_t k) { return !(G.ordRec[k].x < S); });
+        if (tid == 0) s_p = p;
+    }
     if (tid == 0)
     {
         s_ctr = *ctr;
-        s_p = win_lower_bound(G.ordRec, G.nsorted, S);
         s_V = S;
         s_cnext = w + 1;
         s_m = 0;
@@ -1216,11 +1247,36 @@ __device__ int win_sweep_replay(const WinGrid& G, int w, const SweepBufs& B, flo
         if (s_m == 0)
         {
             // ---- FIFO empty: one heap pop by the sequential rules ----
+            // (the list's head found 512 positions at a time, the cuts by a
+            // warp, the neighbours a lane each: one thread doing all of it
+            // took 28,000 cycles)
             if (tid == 0)
             {
-                std::int64_t p = s_p;
-                while (p < G.nsorted && !(G.ordRec[p].y < S)) ++p;
-                s_p = p;
+                s_first = ~0ull;
+                s_lc = kWinNone;
+            }
+            if (s_p < lst.base || s_p >= lst.base + kSwThreads)
+            {
+                lst.base = s_p;
+                lst.load(G, tid);
+            }
+            __syncthreads();
+            for (;;)
+            {
+                const std::int64_t q0 = lst.base + tid;
+                const bool head = q0 >= s_p && q0 < G.nsorted && lst.o.y < S;
+                const unsigned hb = __ballot_sync(0xffffffffu, head);
+                if (head && static_cast<int>(tid & 31) == __ffs(hb) - 1)
+                    atomicMin(&s_first, static_cast<unsigned long long>(q0));
+                const bool more = lst.base + kSwThreads < G.nsorted;
+                if (__syncthreads_or(head) || !more) break;
+                lst.base += kSwThreads;
+                lst.load(G, tid);
+            }
+            if (s_first == static_cast<unsigned long long>(lst.base + tid))
+            {
+                s_lz = lst.o.x;
+                s_lc = __float_as_uint(lst.o.z);
             }
             // the least discovered heap cell: in the first non-empty list
             // (every near key is below T, and every level's keys below the
@@ -1263,119 +1319,124 @@ __device__ int win_sweep_replay(const WinGrid& G, int w, const SweepBufs& B, flo
                 sh.red_s[tid >> 5] = bslot;
             }
             __syncthreads();
-            if (tid == 0)
+            if (tid < 32)
             {
-                for (int k = 1; k < kSwThreads / 32; ++k)
-                    if (win_key_less(sh.red_v[k], sh.red_i[k], bz, bi))
-                    {
-                        bz = sh.red_v[k];
-                        bi = sh.red_i[k];
-                        bslot = sh.red_s[k];
-                    }
-                const bool have_l = s_p < G.nsorted;
-                float hz = INFINITY;
-                std::uint32_t hc = kWinNone;
-                bool from_list = false;
-                if (have_l)
+                const int lane = tid;
+                bz = lane < kSwThreads / 32 ? sh.red_v[lane] : INFINITY;
+                bi = lane < kSwThreads / 32 ? sh.red_i[lane] : kWinNone;
+                bslot = lane < kSwThreads / 32 ? sh.red_s[lane] : kWinNone;
+                for (int o = 16; o > 0; o >>= 1)
                 {
-                    const float4 o = G.ordRec[s_p];
-                    hz = o.x;
-                    hc = __float_as_uint(o.z);
-                    from_list = true;
+                    const float oz = __shfl_xor_sync(0xffffffffu, bz, o);
+                    const std::uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                    const std::uint32_t os = __shfl_xor_sync(0xffffffffu, bslot, o);
+                    if (win_key_less(oz, oi, bz, bi))
+                    {
+                        bz = oz;
+                        bi = oi;
+                        bslot = os;
+                    }
                 }
+                const bool have_l = s_lc != kWinNone;
+                float hz = have_l ? s_lz : INFINITY;
+                std::uint32_t hc = s_lc;
+                bool from_list = have_l;
                 if (bi != kWinNone && (!have_l || win_key_less(bz, bi, hz, hc)))
                 {
                     hz = bz;
                     hc = bi;
                     from_list = false;
                 }
-                if (hc == kWinNone)
-                {
-                    s_next = G.ncut;
-                    s_stop = 1;
-                }
+                const std::int64_t p = have_l ? static_cast<std::int64_t>(s_first) : G.nsorted;
+                float V = s_V;
+                int cn = s_cnext;
+                bool stop = hc == kWinNone;
+                if (stop) cn = G.ncut;
                 else
                 {
-                    const float V = s_V;
                     // first cut above V (sweeps leave it to this point)
-                    {
-                        int lo = s_cnext, hi = G.ncut;
-                        while (lo < hi)
-                        {
-                            const int mid = (lo + hi) >> 1;
-                            if (G.cuts[mid] <= V) lo = mid + 1;
-                            else hi = mid;
-                        }
-                        s_cnext = lo;
-                    }
-                    const int cn = s_cnext;
+                    cn = sw_search<int>(cn, G.ncut, [&](int k) { return G.cuts[k] > V; });
                     const bool trig = hz <= V && cn > 0 && G.cuts[cn - 1] >= hz;
-                    if (!trig && (cn >= G.ncut || G.cand[cn]))
+                    stop = !trig && (cn >= G.ncut || G.cand[cn]);
+                }
+                if (lane == 0)
+                {
+                    s_p = (!stop && from_list) ? p + 1 : p;
+                    if (stop)
                     {
                         s_next = cn;
                         s_stop = 1;
                     }
-                    else
+                }
+                if (!stop)
+                {
+                    // the pop's open neighbours, a lane each
+                    const int r = win_row(hc, G.nc, 1.0f / static_cast<float>(G.nc));
+                    const int c = static_cast<int>(hc - static_cast<std::uint32_t>(r) * G.nc);
+                    std::uint32_t j = kWinNone;
+                    float zj = 0.0f;
+                    int rr, cc;
+                    if (lane < 8 && fill_nb(G.nr, G.nc, G.per_ns, G.per_ew, r, c, lane, rr, cc))
                     {
-                        if (from_list) ++s_p;
+                        j = static_cast<std::uint32_t>(rr) * G.nc + cc;
+                        if (!open_cell(j, zj)) j = kWinNone;
+                    }
+                    // (a cell reached twice across a short wrapped axis counts once)
+                    for (int k = 0; k < 7; ++k)
+                    {
+                        const std::uint32_t other = __shfl_sync(0xffffffffu, j, k);
+                        if (lane > k && j != kWinNone && other == j) j = kWinNone;
+                    }
+                    const bool raised = j != kWinNone && zj <= hz;
+                    const int lv = (j == kWinNone || raised) ? -2 : (zj < s_T ? -1 : level_of(zj));
+                    const unsigned rb = __ballot_sync(0xffffffffu, raised);
+                    const unsigned lower = (1u << lane) - 1u;
+                    // the popped heap cell leaves its list: the last entry takes its place
+                    if (lane == 0 && !from_list)
+                    {
+                        if (which < 0)
+                        {
+                            const std::uint32_t last = --s_nd;
+                            dc[bslot] = dc[last];
+                            dk[bslot] = dk[last];
+                        }
                         else
                         {
-                            if (which < 0)
-                            {
-                                const std::uint32_t last = --s_nd;
-                                dc[bslot] = dc[last];
-                                dk[bslot] = dk[last];
-                            }
-                            else
-                            {
-                                const std::uint32_t last = --s_nl[which];
-                                std::uint32_t* wc = lvc(which);
-                                float* wk = lvk(which);
-                                wc[bslot] = wc[last];
-                                wk[bslot] = wk[last];
-                            }
+                            const std::uint32_t last = --s_nl[which];
+                            std::uint32_t* wc = lvc(which);
+                            float* wk = lvk(which);
+                            wc[bslot] = wc[last];
+                            wk[bslot] = wk[last];
                         }
-                        if (hz > s_V)
+                    }
+                    __syncwarp();
+                    if (raised)
+                    {
+                        const std::uint32_t m = __popc(rb & lower);
+                        sh.fc[m] = j;
+                        sh.fv[m] = raise_from(hz, G.eps, (lane & 1) ? G.Ld : G.L);
+                    }
+                    for (int k = -1; k < kSwLv; ++k)
+                    {
+                        const unsigned b = __ballot_sync(0xffffffffu, lv == k);
+                        if (!b) continue;
+                        std::uint32_t* ctr = k < 0 ? &s_nd : &s_nl[k];
+                        const std::uint32_t at = *ctr + __popc(b & lower);
+                        if (lv == k)
                         {
-                            s_V = hz;
-                            while (s_cnext < G.ncut && G.cuts[s_cnext] <= s_V) ++s_cnext;
+                            (k < 0 ? dc : lvc(k))[at] = j;
+                            (k < 0 ? dk : lvk(k))[at] = zj;
                         }
-                        const int r = static_cast<int>(hc / static_cast<std::uint32_t>(G.nc));
-                        const int c = static_cast<int>(hc - static_cast<std::uint32_t>(r) * G.nc);
-                        std::uint32_t m = 0;
-                        for (int d = 0; d < 8; ++d)
-                        {
-                            int rr, cc;
-                            if (!fill_nb(G.nr, G.nc, G.per_ns, G.per_ew, r, c, d, rr, cc)) continue;
-                            const std::uint32_t j = static_cast<std::uint32_t>(rr) * G.nc + cc;
-                            float zj;
-                            if (!open_cell(j, zj)) continue;
-                            if (zj <= hz)
-                            {
-                                sh.fc[m] = j;
-                                sh.fv[m] = raise_from(hz, G.eps, (d & 1) ? G.Ld : G.L);
-                                ++m;
-                                set_queued(j);
-                            }
-                            else
-                            {
-                                if (zj < s_T)
-                                {
-                                    dc[s_nd] = j;
-                                    dk[s_nd] = zj;
-                                    ++s_nd;
-                                }
-                                else
-                                {
-                                    const int k = level_of(zj);
-                                    lvc(k)[s_nl[k]] = j;
-                                    lvk(k)[s_nl[k]] = zj;
-                                    ++s_nl[k];
-                                }
-                                set_queued(j);
-                            }
-                        }
-                        s_m = m;
+                        __syncwarp();
+                        if (lane == 0) *ctr += __popc(b);
+                        __syncwarp();
+                    }
+                    if (j != kWinNone) set_queued(j);
+                    if (lane == 0)
+                    {
+                        s_cnext = cn;
+                        s_V = fmaxf(V, hz);
+                        s_m = __popc(rb);
                     }
                 }
             }

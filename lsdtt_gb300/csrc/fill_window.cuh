@@ -250,7 +250,8 @@ struct WinResult
 };
 
 // Replay the window starting at cut w, by one full warp (all 32 lanes call
-// it with the same arguments). `pop_limit` bounds the pops (0: none). Every
+// it with the same arguments). `pop_limit` bounds the pops (0: none); a replay
+// whose result is no longer wanted stops once *quit is set. Every
 // loop iteration takes one entry from the list, the heap or the FIFO or
 // leaves; each cell enters the heap or the FIFO at most once (the seen set),
 // so the replay ends after at most nsorted + (cells seen) iterations.
@@ -259,7 +260,8 @@ struct WinResult
 // that chain: the neighbour loads are issued before the heap is repaired,
 // and the cuts around the running maximum and a block of the sorted list sit
 // in registers (one entry per lane).
-__device__ WinResult win_replay(const WinGrid& G, int w, const WinStore& s, std::uint64_t pop_limit)
+__device__ WinResult win_replay(const WinGrid& G, int w, const WinStore& s, std::uint64_t pop_limit,
+                                const unsigned* quit = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -464,6 +466,11 @@ __device__ WinResult win_replay(const WinGrid& G, int w, const WinStore& s, std:
                     cand_l = G.cand[cb + lane] != 0;
                 }
             }
+        }
+        if (quit && (pops & 31) == 31 && *reinterpret_cast<const volatile unsigned*>(quit))
+        {
+            res.status = kWinOverflow;
+            break;
         }
         if (pop_limit && ++pops > pop_limit)
         {
