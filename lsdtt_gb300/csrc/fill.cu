@@ -73,76 +73,35 @@ __global__ void __launch_bounds__(256) fill_relax(int nr, int nc, bool per_ns, b
                     blockIdx.y, gridDim.x, gridDim.y);
 }
 
-// Active tiles of a pass, one thread per tile: tile (tx, ty) is active when
-// it or one of its eight neighbours (periodic axes wrap) changed in the
-// previous pass. Clears dirty_out (an active tile's relaxation sets it
-// again) and appends the active tiles to the list of their colour
-// (list + colour * cap, warp-aggregated), counting them (cnt[colour]) and
-// their cells (cnt[kFillColours]).
-__global__ void fill_active(int nr, int nc, bool per_ns, bool per_ew, int ntx, int nty,
-                            const std::uint8_t* __restrict__ din, std::uint8_t* __restrict__ dout,
-                            std::int32_t* __restrict__ list, std::int64_t cap, unsigned long long* __restrict__ cnt)
+__global__ void fill_queue_init(int tiles, TileQueue Q)
 {
     LSDTT_COUNT();
-    const std::int32_t t = static_cast<std::int32_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    bool active = false;
-    unsigned cells = 0;
-    int colour = -1;
-    if (t < ntx * nty)
-    {
-        const int tx = t % ntx, ty = t / ntx;
-        for (int dy = -1; dy <= 1 && !active; ++dy)
-            for (int dx = -1; dx <= 1; ++dx)
-            {
-                int yy = ty + dy, xx = tx + dx;
-                if (per_ns) yy = (yy + nty) % nty;
-                if (per_ew) xx = (xx + ntx) % ntx;
-                if (yy < 0 || yy >= nty || xx < 0 || xx >= ntx) continue;
-                if (din[yy * ntx + xx])
-                {
-                    active = true;
-                    break;
-                }
-            }
-        dout[t] = 0;
-        if (active)
-        {
-            cells = static_cast<unsigned>(min(kT, nr - ty * kT)) * static_cast<unsigned>(min(kT, nc - tx * kT));
-            colour = fill_colour(tx, ty, ntx, nty, per_ns, per_ew);
-        }
-    }
-    const int lane = threadIdx.x & 31;
-    const unsigned peers = __match_any_sync(0xffffffffu, colour);
-    const int leader = __ffs(peers) - 1;
-    unsigned long long base = 0;
-    if (active && lane == leader) base = atomicAdd(&cnt[colour], static_cast<unsigned long long>(__popc(peers)));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (active) list[colour * cap + static_cast<std::int64_t>(base) + __popc(peers & ((1u << lane) - 1u))] = t;
-    for (int o = 16; o > 0; o >>= 1) cells += __shfl_down_sync(0xffffffffu, cells, o);
-    if (lane == 0 && cells) atomicAdd(&cnt[kFillColours], static_cast<unsigned long long>(cells));
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 3) Q.cnt[t] = t == 0 ? static_cast<unsigned>(tiles) : 0u;
+    if (t >= tiles) return;
+    Q.list[0][t] = t;
+    Q.queued[t] = 1u;
 }
 
-// Relaxation of one colour's listed active tiles by a persistent grid (block
-// w takes entries w, w + grid, ...), the tile gate skipped: one block per
-// tile spent most of a late pass on inactive tiles reading their
-// neighbours' flags.
-__global__ void __launch_bounds__(256) fill_relax_list(int nr, int nc, bool per_ns, bool per_ew, float L, float Ld,
-                                                       float min_slope, const float* __restrict__ z,
-                                                       const std::uint8_t* __restrict__ kind, float* __restrict__ F,
-                                                       int* __restrict__ changed,
-                                                       const std::uint8_t* __restrict__ dirty_in,
-                                                       std::uint8_t* __restrict__ dirty_out, int ntx, int nty,
-                                                       const std::int32_t* __restrict__ list,
-                                                       const unsigned long long* __restrict__ count)
+// A pass over the queued tiles by a persistent grid (block w takes entries w,
+// w + grid, ...).
+template <bool kStep>
+__global__ void __launch_bounds__(256) fill_scan_pass(int nr, int nc, bool per_ns, bool per_ew, float L, float Ld,
+                                                      float eps, const float* __restrict__ z,
+                                                      const std::uint8_t* __restrict__ kind, float* F, int ntx, int nty,
+                                                      TileQueue Q, int pass)
 {
     LSDTT_COUNT();
-    const std::int64_t n = static_cast<std::int64_t>(*count);
-    for (std::int64_t w = blockIdx.x; w < n; w += gridDim.x)
+    __shared__ ScanTile S;
+    const std::int32_t* list = (pass & 1) ? Q.list[1] : Q.list[0];
+    std::int32_t* next = (pass & 1) ? Q.list[0] : Q.list[1];
+    const unsigned n = Q.cnt[pass % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) Q.cnt[(pass + 2) % 3] = 0u;
+    for (unsigned w = blockIdx.x; w < n; w += gridDim.x)
     {
         const int t = list[w];
-        fill_relax_tile(nr, nc, per_ns, per_ew, L, Ld, min_slope, z, kind, F, changed, dirty_in, dirty_out, t % ntx,
-                        t / ntx, ntx, nty, false);
-        __syncthreads();  // the tile's shared arrays are staged again for the next tile
+        fill_scan_tile<kStep>(S, nr, nc, per_ns, per_ew, L, Ld, eps, z, kind, F, t % ntx, t / ntx, ntx, nty, Q, next,
+                              Q.cnt + (pass + 1) % 3);
     }
 }
 
@@ -155,69 +114,61 @@ namespace
 {
 
 // The relaxation from fill_init to its fixed point with raise step `eps`
-// (0: the epsilon-0 fill) into F. Work buffers are the caller's.
+// (0: the epsilon-0 fill) into F. Work buffers are the caller's; `queue` holds
+// three words a tile and three counts.
 cudaError_t relax_fill(int nr, int nc, bool per_ns, bool per_ew, float L, float Ld, float eps, const float* z_dev,
                        const std::uint8_t* mask_dev, double nodata, float* F, std::uint8_t* kind, int* flags,
-                       int* hflag, std::uint8_t* dirty, std::int32_t* list, unsigned long long* cnt,
-                       unsigned long long* hcnt, cudaStream_t st, bool* converged)
+                       std::uint32_t* queue, cudaStream_t st, bool* converged)
 {
     *converged = false;
     const std::int64_t n = static_cast<std::int64_t>(nr) * nc;
-    const std::int64_t ntiles = static_cast<std::int64_t>((nc + kT - 1) / kT) * ((nr + kT - 1) / kT);
+    const int ntx = (nc + kT - 1) / kT, nty = (nr + kT - 1) / kT, ntiles = ntx * nty;
     cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(int) * 2, st);
-    cudaMemsetAsync(dirty, 1, static_cast<std::size_t>(2 * ntiles), st);
     fill_interior_nodata<<<grid_blocks(n, 256), 256, 0, st>>>(nr, nc, z_dev, mask_dev, nodata, flags);
     fill_init<<<grid_blocks(n, 256), 256, 0, st>>>(nr, nc, per_ns, per_ew, z_dev, mask_dev, nodata, flags, F, kind);
-    const dim3 block(32, 8);
-    const dim3 tiles((nc + kT - 1) / kT, (nr + kT - 1) / kT);
-    // Global passes until no tile changes; the change flag is read back every
-    // few passes to keep the host out of the loop.
+    TileQueue Q{};
+    Q.list[0] = reinterpret_cast<std::int32_t*>(queue);
+    Q.list[1] = reinterpret_cast<std::int32_t*>(queue + ntiles);
+    Q.queued = queue + 2 * static_cast<std::size_t>(ntiles);
+    Q.cnt = queue + 3 * static_cast<std::size_t>(ntiles);
+    fill_queue_init<<<grid_blocks(std::max(ntiles, 3), 256), 256, 0, st>>>(ntiles, Q);
+    // Passes until the queue is empty; its counts are read back every few
+    // passes to keep the host out of the loop.
     const int kCheckEvery = 4;
     const long max_pass = 4L * (nr + nc) + 64;  // bound: any path crosses each tile row/column at most a few times
-    const int ntx = static_cast<int>(tiles.x), nty = static_cast<int>(tiles.y);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned list_grid = static_cast<unsigned>(std::max(1, sms) * 8);
-    const unsigned colours = fill_colour_mask(ntx, nty, per_ns, per_ew);
-    long pass = 0;
+    const unsigned grid = static_cast<unsigned>(std::min(ntiles, std::max(1, sms) * 6));
+    int pass = 0;
+    unsigned cnt[3] = {0, 0, 0};
     while (e == cudaSuccess)
     {
-        cudaMemsetAsync(flags + 1, 0, sizeof(int), st);
         for (int k = 0; k < kCheckEvery && e == cudaSuccess; ++k, ++pass)
         {
-            // Each pass lists its active tiles by colour, then relaxes each
-            // colour's in turn. Algorithmic bytes per pass: z 4 + mask 1
-            // in, filled value 4 out per relaxed cell (counted when
-            // profiling).
-            const std::uint8_t* din = dirty + (pass & 1) * ntiles;
-            std::uint8_t* dout = dirty + ((pass + 1) & 1) * ntiles;
-            cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * (kFillColours + 1), st);
-            fill_active<<<grid_blocks(ntiles, 256), 256, 0, st>>>(nr, nc, per_ns, per_ew, ntx, nty, din, dout, list,
-                                                                   ntiles, cnt);
+            // Algorithmic bytes: z 4 + mask 1 in, filled value 4 out per cell
+            // of a queued tile (counted when profiling).
             double bytes = 9.0 * static_cast<double>(n);
             if (profiling_enabled())
             {
-                cudaMemcpyAsync(hcnt, cnt, sizeof(unsigned long long) * (kFillColours + 1), cudaMemcpyDeviceToHost,
-                                st);
+                cudaMemcpyAsync(cnt, Q.cnt, sizeof(cnt), cudaMemcpyDeviceToHost, st);
                 e = cudaStreamSynchronize(st);
-                bytes = 9.0 * static_cast<double>(hcnt[kFillColours]);
+                bytes = std::min(bytes, 9.0 * kT * kT * static_cast<double>(cnt[pass % 3]));
             }
             LSDTT_TIMED("fill_relax", bytes, st, ({
-                            for (int c = 0; c < kFillColours; ++c)
-                            {
-                                if (!((colours >> c) & 1u)) continue;
-                                fill_relax_list<<<list_grid, block, 0, st>>>(nr, nc, per_ns, per_ew, L, Ld, eps, z_dev,
-                                                                             kind, F, flags + 1, din, dout, ntx, nty,
-                                                                             list + c * ntiles, cnt + c);
-                            }
+                            if (eps > 0.0f)
+                                fill_scan_pass<true><<<grid, 256, 0, st>>>(nr, nc, per_ns, per_ew, L, Ld, eps, z_dev, kind,
+                                                                           F, ntx, nty, Q, pass);
+                            else
+                                fill_scan_pass<false><<<grid, 256, 0, st>>>(nr, nc, per_ns, per_ew, L, Ld, 0.0f, z_dev,
+                                                                            kind, F, ntx, nty, Q, pass);
                         }));
         }
         if (e != cudaSuccess) break;
-        cudaMemcpyAsync(hflag, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-        e = cudaStreamSynchronize(st);
+        e = cudaMemcpyAsync(cnt, Q.cnt, sizeof(cnt), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) break;
-        if (*hflag == 0)
+        if (cnt[pass % 3] == 0)
         {
             *converged = true;
             break;
@@ -346,46 +297,34 @@ extern "C" int lsdtt_gpu_fill_pits(const lsdtt_gpu_grid* grid, const float* z_de
     if (eps > 0.0f && n > (std::int64_t(1) << 31))
         return fail(LSDTT_GPU_EINVAL, "lsdtt_gpu_fill_pits: grids above 2^31 cells are not supported with min_slope > 0");
     std::uint8_t* kind = nullptr;
-    int* flags = nullptr;   // [0] interior nodata, [1] changed
-    int* hflag = nullptr;
-    std::uint8_t* dirty = nullptr;  // two per-tile activity planes
-    std::int32_t* list = nullptr;   // active tiles of the current pass, by colour
-    unsigned long long* cnt = nullptr;  // their count and cells
-    unsigned long long* hcnt = nullptr;
-    float* F0 = nullptr;            // epsilon-0 fill (min_slope > 0 only)
+    int* flags = nullptr;             // [0] interior nodata
+    std::uint32_t* queue = nullptr;   // tile queue of the relaxation
+    float* F0 = nullptr;              // epsilon-0 fill (min_slope > 0 only)
     const std::int64_t ntiles = static_cast<std::int64_t>((nc + kT - 1) / kT) * ((nr + kT - 1) / kT);
     cudaError_t e = cudaMallocAsync(&kind, static_cast<std::size_t>(n), st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&dirty, static_cast<std::size_t>(2 * ntiles), st);
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&list, sizeof(std::int32_t) * kFillColours * static_cast<std::size_t>(ntiles), st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&cnt, sizeof(unsigned long long) * (kFillColours + 1), st);
+        e = cudaMallocAsync(&queue, sizeof(std::uint32_t) * (3 * static_cast<std::size_t>(ntiles) + 4), st);
     if (e == cudaSuccess) e = cudaMallocAsync(&flags, sizeof(int) * 2, st);
     if (e == cudaSuccess && eps > 0.0f) e = cudaMallocAsync(&F0, sizeof(float) * static_cast<std::size_t>(n), st);
-    if (e == cudaSuccess) e = cudaMallocHost(&hflag, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&hcnt, sizeof(unsigned long long) * (kFillColours + 1));
     const float L = static_cast<float>(grid->cell_size);
     const float Ld = L * static_cast<float>(1.4142135623730950488);
     bool converged = true;
     unsigned failure = 0;
     if (e == cudaSuccess)
         e = relax_fill(nr, nc, per_ns, per_ew, L, Ld, eps, z_dev, mask_dev, grid->no_data_value, out_dev, kind, flags,
-                       hflag, dirty, list, cnt, hcnt, st, &converged);
+                       queue, st, &converged);
     if (e == cudaSuccess && converged && eps > 0.0f)
     {
         e = relax_fill(nr, nc, per_ns, per_ew, L, Ld, 0.0f, z_dev, mask_dev, grid->no_data_value, F0, kind, flags,
-                       hflag, dirty, list, cnt, hcnt, st, &converged);
+                       queue, st, &converged);
         if (e == cudaSuccess && converged)
             e = exact_fill_single(nr, nc, per_ns, per_ew, L, Ld, eps, static_cast<float>(grid->no_data_value), z_dev,
                                   kind, F0, out_dev, st, &failure);
     }
     cudaFreeAsync(kind, st);
-    cudaFreeAsync(dirty, st);
-    cudaFreeAsync(list, st);
-    cudaFreeAsync(cnt, st);
+    cudaFreeAsync(queue, st);
     cudaFreeAsync(flags, st);
     cudaFreeAsync(F0, st);
-    cudaFreeHost(hflag);
-    cudaFreeHost(hcnt);
     if (e != cudaSuccess) return cuda_fail(e, "lsdtt_gpu_fill_pits");
     if (!converged) return fail(LSDTT_GPU_ETIMEOUT, "lsdtt_gpu_fill_pits: relaxation did not converge");
     if (failure)

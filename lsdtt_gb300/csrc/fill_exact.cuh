@@ -587,6 +587,11 @@ constexpr int kExB_FQ = 128, kExB_DH = 4096, kExB_HS = 8192, kExB_OC = 1024;
 // 32.4, 36.7, 49.1 ms; always replayed first, a 512 x 512 noise tilt takes
 // 27.7 ms and not 22.3.)
 constexpr unsigned kExMinWindows = 20;
+// Pops after which the small size leaves a window to the replays beside the
+// chain, which waits for the small size only. (32, 96, 192, no limit: a
+// 97 x 131 noise tilt 3.18, 3.24, 3.36, 3.74 ms, a 1500 x 1403 pitted fractal
+// 152.7, 153.4, 153.2, 154.3.)
+constexpr unsigned long long kExSidePops = 32;
 constexpr std::size_t kExSmemA = 8 * kExA_FQ + 8 * (kExA_DH + 2) + 4 * kExA_HS + 8 * kExA_OC;
 constexpr std::size_t kExSmemM = 8 * kExM_FQ + 8 * (kExM_DH + 2) + 4 * kExM_HS + 8 * kExM_OC;
 constexpr std::size_t kExSmemB = 8 * kExB_FQ + 8 * (kExB_DH + 2) + 4 * kExB_HS + 8 * kExB_OC;
@@ -725,7 +730,7 @@ inline cudaError_t ex_run(const ExMember* mem, const std::uint16_t* blk_member, 
     };
     LSDTT_TIMED(nm[4], 16.0 * cells, st,
                 (ex_windows<kExA_FQ, kExA_DH, kExA_HS, kExA_OC><<<sms * 20, 32, kExSmemA, st>>>(
-                    mem, z, kind, F0, B, B.wl, B.u + 1, B.u + 2, static_cast<unsigned long long>(N), 16ull * kExA_HS,
+                    mem, z, kind, F0, B, B.wl, B.u + 1, B.u + 2, static_cast<unsigned long long>(N), side ? kExSidePops : 16ull * kExA_HS,
                     0u, nullptr)));
     if (side && e == cudaSuccess)
     {
