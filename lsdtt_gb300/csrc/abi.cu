@@ -79,14 +79,34 @@ bool device_ok()
 namespace
 {
 
-__global__ void check_valid_z(const float* __restrict__ z, const std::uint8_t* __restrict__ mask, std::int64_t n,
-                              float ndv, unsigned long long* __restrict__ first_bad)
+// The engine's copy of the mask (0 or 1) and the first valid cell whose
+// elevation is not finite or is the nodata value. Eight cells a thread, all
+// their loads in flight: as a copy and a check of one cell a thread each, block
+// starts bounded both (16.4 M cells 46 + 60 us, now 23).
+constexpr int kInputPer = 8;
+
+__global__ void __launch_bounds__(256) check_inputs(const float* __restrict__ z, const std::uint8_t* __restrict__ in,
+                                                    std::int64_t n, float ndv, std::uint8_t* __restrict__ mask,
+                                                    unsigned long long* __restrict__ first_bad)
 {
     LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n || !mask[i]) return;
-    const float v = z[i];
-    if (!isfinite(v) || v == ndv) atomicMin(first_bad, static_cast<unsigned long long>(i));
+    const std::int64_t base = static_cast<std::int64_t>(blockIdx.x) * (256 * kInputPer) + threadIdx.x;
+    float v[kInputPer];
+    std::uint8_t m[kInputPer];
+#pragma unroll
+    for (int k = 0; k < kInputPer; ++k)
+    {
+        const std::int64_t i = base + 256 * k;
+        v[k] = i < n ? z[i] : 0.0f;
+        m[k] = i < n ? in[i] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kInputPer; ++k)
+    {
+        const std::int64_t i = base + 256 * k;
+        if (i < n) mask[i] = m[k] ? 1 : 0;
+        if (m[k] && (!isfinite(v[k]) || v[k] == ndv)) atomicMin(first_bad, static_cast<unsigned long long>(i));
+    }
 }
 
 __global__ void check_finite_w(const double* __restrict__ w, const std::uint8_t* __restrict__ mask, std::int64_t n,
@@ -96,13 +116,6 @@ __global__ void check_finite_w(const double* __restrict__ w, const std::uint8_t*
     const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n || !mask[i]) return;
     if (!isfinite(w[i])) atomicMin(first_bad, static_cast<unsigned long long>(i));
-}
-
-__global__ void copy_mask(const std::uint8_t* __restrict__ in, std::int64_t n, std::uint8_t* __restrict__ out)
-{
-    LSDTT_COUNT();
-    const std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[i] ? 1 : 0;
 }
 
 __global__ void stamp_forced(const std::int64_t* __restrict__ forced, std::int64_t nf, std::int64_t n,
@@ -337,8 +350,8 @@ int lsdtt_gpu_flow_build(lsdtt_gpu_flow* f, const float* z_dev, const std::uint8
     // derr[3] = first bad forced-outlet entry.
     unsigned long long init[4] = {0ull, ~0ull, 0ull, ~0ull};
     cudaMemcpyAsync(f->derr, init, sizeof(init), cudaMemcpyHostToDevice, st);
-    copy_mask<<<nb, 256, 0, st>>>(mask_dev, n, f->mask);
-    check_valid_z<<<nb, 256, 0, st>>>(z_dev, f->mask, n, static_cast<float>(g.nodata), f->derr + 1);
+    check_inputs<<<grid_blocks(n, 256 * kInputPer), 256, 0, st>>>(z_dev, mask_dev, n, static_cast<float>(g.nodata),
+                                                                  f->mask, f->derr + 1);
     std::uint8_t* plane = nullptr;
     if (n_forced > 0 && forced_dev)
     {
