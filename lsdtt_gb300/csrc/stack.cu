@@ -801,31 +801,141 @@ __global__ void accum_seed(Grid g, const std::uint8_t* __restrict__ mask, const 
     out[c] = mask[c] ? (w ? w[c] : dw) : 0.0;
 }
 
-__global__ void accum_level(Grid g, const std::uint8_t* __restrict__ mask, const std::uint8_t* __restrict__ dir,
-                            const std::int64_t* __restrict__ topo, const std::uint32_t* __restrict__ topo_pos,
-                            std::int64_t lo, std::int64_t hi, double* __restrict__ acc)
+// A cell's donors in topological order, as one word: their number (bits 0-3)
+// and 3 bits of direction each, and whether it is on the grid's edge. It is formed for all cells at once, so a level
+// waits for its additions only, not for the search, the positions and the sort
+// before them.
+constexpr std::uint32_t kAccumEdge = 1u << 28;
+
+__global__ void __launch_bounds__(256) accum_codes(Grid g, const std::uint8_t* __restrict__ dir,
+                                                   const std::int64_t* __restrict__ topo,
+                                                   const std::uint32_t* __restrict__ topo_pos, std::int64_t lo,
+                                                   std::int64_t nv, std::uint32_t* __restrict__ code)
 {
     LSDTT_COUNT();
     const std::int64_t i = lo + static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= hi) return;
+    if (i >= nv) return;
     const std::int64_t c = topo[i];
-    std::int64_t d[8];
-    const int k = donor_list(g, mask, dir, c, d);
-    // Order donors by topological position.
-    std::uint32_t p[8];
-    for (int a = 0; a < k; ++a) p[a] = topo_pos[d[a]];
-    for (int a = 1; a < k; ++a)
+    const int row = static_cast<int>(c / g.nc), col = static_cast<int>(c % g.nc);
+    const bool inner = is_interior(g, row, col);
+    std::uint64_t key[8];  // position << 3 | direction; all ones: no donor
+    unsigned k = 0;
+#pragma unroll
+    for (int d = 0; d < 8; ++d)
     {
-        const std::uint32_t pk = p[a];
-        const std::int64_t dk = d[a];
-        int j = a;
-        while (j > 0 && p[j - 1] > pk) { p[j] = p[j - 1]; d[j] = d[j - 1]; --j; }
-        p[j] = pk;
-        d[j] = dk;
+        std::int64_t nf = c + static_cast<std::int64_t>(d8_dr(d)) * g.nc + d8_dc(d);
+        if (!inner)
+        {
+            const Step s = resolve_step(g, row, col, d);
+            nf = s.kind == 1 ? static_cast<std::int64_t>(s.r) * g.nc + s.c : c;
+        }
+        // (a masked cell has no direction, and c's own does not lead to c)
+        const bool donor = nf != c && dir[nf] == ((d + 4) & 7);
+        key[d] = donor ? (static_cast<std::uint64_t>(topo_pos[nf]) << 3) | static_cast<unsigned>(d) : ~0ull;
+        k += donor ? 1u : 0u;
+    }
+    // odd-even transposition sort of the eight keys, in registers
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int j = r & 1; j + 1 < 8; j += 2)
+        {
+            const std::uint64_t x = key[j], y = key[j + 1];
+            key[j] = x < y ? x : y;
+            key[j + 1] = x < y ? y : x;
+        }
+    std::uint32_t w = k | (inner ? 0u : kAccumEdge);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w |= static_cast<std::uint32_t>(key[j] & 7u) << (4 + 3 * j);
+    code[i] = w;
+}
+
+__device__ __forceinline__ void accum_cell(const Grid& g, std::int64_t c, std::uint32_t w, double* acc)
+{
+    const int k = static_cast<int>(w & 15u);
+    if (k == 0) return;
+    double v[8];
+    if (w & kAccumEdge)
+    {
+        const int row = static_cast<int>(c / g.nc), col = static_cast<int>(c % g.nc);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+            if (j >= k) break;
+            const Step s = resolve_step(g, row, col, static_cast<int>((w >> (4 + 3 * j)) & 7u));
+            v[j] = acc[static_cast<std::int64_t>(s.r) * g.nc + s.c];
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+            if (j >= k) break;
+            const int d = static_cast<int>((w >> (4 + 3 * j)) & 7u);
+            v[j] = acc[c + static_cast<std::int64_t>(d8_dr(d)) * g.nc + d8_dc(d)];
+        }
     }
     double s = acc[c];
-    for (int a = 0; a < k; ++a) s = __dadd_rn(s, acc[d[a]]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+    {
+        if (j >= k) break;
+        s = __dadd_rn(s, v[j]);
+    }
     acc[c] = s;
+}
+
+__global__ void __launch_bounds__(128) accum_level(Grid g, const std::int64_t* __restrict__ topo,
+                                                   const std::uint32_t* __restrict__ code, std::int64_t lo,
+                                                   std::int64_t hi, double* acc)
+{
+    LSDTT_COUNT();
+    const std::int64_t i = lo + static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < hi) accum_cell(g, topo[i], code[i], acc);
+}
+
+// The levels from k0 on by one block, a barrier between them: a level is no
+// wider than the one below it (each of its cells has a donor there), so once a
+// level fits the block's few passes all later ones do. The next level's cells
+// are fetched while this one adds. 129 x 203 cells, 27 levels: 244 us in 27
+// launches, now 75 in two; 2048 cells and reading the level bounds on the device
+// only (no launch for the widest levels) were no faster.
+constexpr int kAccumTail = 4096;
+
+__global__ void __launch_bounds__(1024) accum_tail(Grid g, const std::int64_t* __restrict__ topo,
+                                                   const std::uint32_t* __restrict__ code,
+                                                   const std::int64_t* __restrict__ start, std::int64_t k0,
+                                                   std::int64_t nlev, double* acc)
+{
+    LSDTT_COUNT();
+    const std::int64_t nv = start[nlev];
+    std::int64_t lo = start[k0], hi = start[k0 + 1];
+    std::int64_t c = 0;
+    std::uint32_t w = 0;
+    if (lo + threadIdx.x < nv)
+    {
+        c = topo[lo + threadIdx.x];
+        w = code[lo + threadIdx.x];
+    }
+    for (std::int64_t k = k0; k < nlev; ++k)
+    {
+        std::int64_t cn = 0;
+        std::uint32_t wn = 0;
+        if (hi + threadIdx.x < nv)
+        {
+            cn = topo[hi + threadIdx.x];
+            wn = code[hi + threadIdx.x];
+        }
+        const std::int64_t next = k + 1 < nlev ? start[k + 2] : hi;
+        if (lo + threadIdx.x < hi) accum_cell(g, c, w, acc);
+        for (std::int64_t i = lo + 1024 + threadIdx.x; i < hi; i += 1024) accum_cell(g, topo[i], code[i], acc);
+        __syncthreads();
+        lo = hi;
+        hi = next;
+        c = cn;
+        w = wn;
+    }
 }
 
 __global__ void level_bounds(const std::int64_t* __restrict__ topo, const std::int32_t* __restrict__ height,
@@ -872,19 +982,23 @@ cudaError_t accumulate(lsdtt_gpu_flow* f, const double* w, double* out, cudaStre
     Scratch& ws = f->ws;
     const std::size_t mark = ws.used;
     std::int64_t* start = ws.take<std::int64_t>(static_cast<std::size_t>(nlev) + 1);
-    if (!start) return cudaErrorMemoryAllocation;
+    std::uint32_t* code = ws.take<std::uint32_t>(static_cast<std::size_t>(nv));
+    if (!start || !code) return cudaErrorMemoryAllocation;
     level_bounds<<<grid_blocks(nv, 256), 256, 0, st>>>(f->topo, f->height, nv, start);
     std::int64_t* hstart = static_cast<std::int64_t*>(std::malloc(sizeof(std::int64_t) * (nlev + 1)));
     if (!hstart) return cudaErrorMemoryAllocation;
     cudaMemcpyAsync(hstart, start, sizeof(std::int64_t) * (nlev + 1), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess)
-        for (std::int64_t k = 1; k < nlev; ++k)  // level 0 cells have no donors
-        {
-            const std::int64_t lo = hstart[k], hi = hstart[k + 1];
-            if (hi > lo) accum_level<<<grid_blocks(hi - lo, 128), 128, 0, st>>>(g, f->mask, f->dir, f->topo,
-                                                                               f->topo_pos, lo, hi, out);
-        }
+    if (e == cudaSuccess && nlev > 1)  // level 0 cells have no donors
+    {
+        const std::int64_t first = hstart[1];
+        accum_codes<<<grid_blocks(nv - first, 256), 256, 0, st>>>(g, f->dir, f->topo, f->topo_pos, first, nv, code);
+        std::int64_t k = 1;
+        for (; k < nlev && hstart[k + 1] - hstart[k] > kAccumTail; ++k)
+            accum_level<<<grid_blocks(hstart[k + 1] - hstart[k], 128), 128, 0, st>>>(g, f->topo, code, hstart[k],
+                                                                                     hstart[k + 1], out);
+        if (k < nlev) accum_tail<<<1, 1024, 0, st>>>(g, f->topo, code, start, k, nlev, out);
+    }
     std::free(hstart);
     ws.used = mark;
     return e != cudaSuccess ? e : cudaGetLastError();
