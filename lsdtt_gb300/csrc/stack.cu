@@ -10,7 +10,7 @@
 //    cell c owns two tour nodes, enter(c) = 2c and exit(c) = 2c+1, and the
 //    successor of every node follows from first child / next sibling /
 //    parent / next outlet.
-// 2. List ranking by a sparse ruling set: every 64th node (plus the head)
+// 2. List ranking by a sparse ruling set: about one node in 32 (and the head)
 //    starts a walk to the next ruler, the rulers' list is ranked
 //    recursively, then every node adds its ruler's rank. With weights
 //    (enter: +1, exit: 0) the prefix is the preorder index; with (+1, -1)
@@ -220,14 +220,30 @@ __device__ __forceinline__ bool node_valid(const RankLevel& L, std::uint32_t v)
     return v < *L.count;
 }
 
-// Per tour node of a ranking level: the ruler whose walk reached it and the
-// two prefixes from that ruler, one 16-byte record (a walk step writes one
-// sector, not three).
+// Per node of a ranking level: the ruler whose walk reached it and the two
+// prefixes from that ruler, one record (a walk step writes one sector, not
+// three). On the tour itself the prefixes are the counts of enter and exit
+// nodes passed, which fit half a word each: a walk that reaches kWalkMax nodes
+// goes on as a ruler of its own.
 struct alignas(16) RankRec
 {
     std::uint32_t owner;
     std::int32_t loc0, loc1, pad;
+    __device__ static RankRec make(std::uint32_t i, int a0, int a1) { return RankRec{i, a0, a1, 0}; }
 };
+struct alignas(8) TourRec
+{
+    std::uint32_t owner;
+    std::uint32_t passed;  // enter nodes | exit nodes << 16
+    // (a0: enter nodes; a1: enter - exit nodes)
+    __device__ static TourRec make(std::uint32_t i, int a0, int a1)
+    {
+        return TourRec{i, static_cast<std::uint32_t>(a0) | static_cast<std::uint32_t>(a0 - a1) << 16};
+    }
+    __device__ int loc0() const { return static_cast<int>(passed & 0xffffu); }
+    __device__ int loc1() const { return static_cast<int>(passed & 0xffffu) - static_cast<int>(passed >> 16); }
+};
+constexpr std::uint32_t kWalkMax = 255;  // nodes of a tour walk before it splits
 
 // Ruler compaction in one pass: each thread takes 16 consecutive nodes, a
 // block scans its rulers and claims a range of the ruler list with one
@@ -235,8 +251,9 @@ struct alignas(16) RankRec
 // counts the level's valid nodes (cnt[2]) for the coverage check.
 constexpr int kCompactPer = 16;
 
+template <class Rec>
 __global__ void __launch_bounds__(256) ruler_compact(RankLevel L, std::uint32_t cap, std::uint32_t* __restrict__ rulers,
-                                                     RankRec* __restrict__ rec, std::uint32_t* __restrict__ cnt)
+                                                     Rec* __restrict__ rec, std::uint32_t* __restrict__ cnt)
 {
     LSDTT_COUNT();
     __shared__ unsigned wsum[8], wval[8], s_base;
@@ -296,42 +313,66 @@ __global__ void __launch_bounds__(256) ruler_compact(RankLevel L, std::uint32_t 
 
 // After the walks: too many rulers, or walks that did not cover every valid
 // node of the level (a successor structure that is not one list).
-__global__ void ruler_checks(const std::uint32_t* cnt, std::uint32_t cap, unsigned long long* err)
+// Adds the rulers that walks split off to the level's count.
+__global__ void ruler_checks(std::uint32_t* cnt, std::uint32_t cap, unsigned long long* err)
 {
     LSDTT_COUNT();
+    cnt[0] += cnt[4];
     if (cnt[0] > cap) raise_error(err, 9, cnt[0]);
     else if (cnt[3] != cnt[2]) raise_error(err, kErrCycle, 2);
 }
 
 // A walk from ruler i to the next ruler. A node of the list is a ruler iff
 // is_ruler(v) or it is the head (ruler_compact), so the stop test needs no
-// load.
-__global__ void ruler_walk(RankLevel L, const std::uint32_t* __restrict__ rulers,
-                           const std::uint32_t* __restrict__ n_rulers, RankRec* __restrict__ rec,
-                           std::int32_t* __restrict__ sub0, std::int32_t* __restrict__ sub1,
-                           std::uint32_t* __restrict__ nxt, std::uint32_t* __restrict__ next_head,
-                           std::uint32_t* __restrict__ walked, std::uint32_t cap,
-                           unsigned long long* __restrict__ err)
+// load. The chain of successors bounds it, so a step loads the next node before
+// it writes this one's record, and a tour walk is split outside the loop (33 M
+// nodes 873 us with both inside, now 458; 16-byte records took 640). One ruler a
+// thread, in the order of the rulers: the walks of a block then keep to the
+// same lines (taking the next ruler as soon as a walk ends spread them, 5.8 ms
+// against 4.0 on an ensemble's tour).
+template <class Rec>
+__global__ void __launch_bounds__(128) ruler_walk(RankLevel L, const std::uint32_t* __restrict__ rulers,
+                                                  std::uint32_t* __restrict__ cnt, Rec* __restrict__ rec,
+                                                  std::int32_t* __restrict__ sub0,
+                                                  std::int32_t* __restrict__ sub1, std::uint32_t* __restrict__ nxt,
+                                                  std::uint32_t* __restrict__ next_head, std::uint32_t cap,
+                                                  unsigned long long* __restrict__ err)
 {
     LSDTT_COUNT();
-    const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const std::uint32_t nr = *n_rulers;
-    if (i >= nr || i >= cap) return;
+    constexpr bool kTour = sizeof(Rec) == sizeof(TourRec);
+    std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const std::uint32_t nr = min(cnt[0], cap);
+    if (i >= nr) return;
     const std::uint32_t head = *L.head;
     std::uint32_t v = rulers[i];
     if (v == head) *next_head = i;
     int a0 = 0, a1 = 0;
-    std::uint32_t steps = 0;
-    do
+    std::uint32_t steps = 0, limit = kTour ? kWalkMax : ~0u;
+    for (;;)
     {
-        rec[v] = RankRec{i, a0, a1, 0};
-        int w0, w1;
-        weights(L, v, w0, w1);
-        a0 += w0;
-        a1 += w1;
-        v = L.succ[v];
-        ++steps;
-    } while (v != kEnd && !is_ruler(v) && v != head && steps <= L.n);
+        do
+        {
+            const std::uint32_t u = L.succ[v];
+            rec[v] = Rec::make(i, a0, a1);
+            int w0, w1;
+            if (kTour) { w0 = 1 - static_cast<int>(v & 1u); w1 = 1 - 2 * static_cast<int>(v & 1u); }
+            else weights(L, v, w0, w1);
+            a0 += w0;
+            a1 += w1;
+            v = u;
+            ++steps;
+        } while (v != kEnd && !is_ruler(v) && v != head && steps <= L.n && steps != limit);
+        if (v == kEnd || is_ruler(v) || v == head || steps > L.n) break;
+        // the walk goes on as ruler j
+        const std::uint32_t j = nr + atomicAdd(&cnt[4], 1u);
+        if (j >= cap) break;  // reported by ruler_checks
+        sub0[i] = a0;
+        sub1[i] = a1;
+        nxt[i] = j;
+        i = j;
+        a0 = a1 = 0;
+        limit += kWalkMax;
+    }
     if (steps > L.n) raise_error(err, kErrCycle, 0);
     sub0[i] = a0;
     sub1[i] = a1;
@@ -340,7 +381,81 @@ __global__ void ruler_walk(RankLevel L, const std::uint32_t* __restrict__ rulers
     // converged group of lanes)
     const unsigned grp = __activemask();
     const unsigned tot = __reduce_add_sync(grp, steps);
-    if ((threadIdx.x & 31) == static_cast<unsigned>(__ffs(grp) - 1)) atomicAdd(walked, tot);
+    if ((threadIdx.x & 31) == static_cast<unsigned>(__ffs(grp) - 1)) atomicAdd(&cnt[3], tot);
+}
+
+// A level of up to kBlockLimit nodes ranked by one block: pointer jumping over
+// the nodes' successors and the sums (and node counts) from a node to the end
+// of the list, in shared memory. The recursion's last levels were five
+// launches each for a few hundred nodes: 52 k tour nodes 100 us after the first
+// level's walk, now 12.
+constexpr std::uint32_t kBlockLimit = 12288;
+constexpr int kBlockPer = 12;  // nodes per thread
+struct BlockNode
+{
+    std::uint32_t next;
+    std::int32_t s0, s1;
+    std::uint32_t count;
+};
+
+__global__ void __launch_bounds__(1024) block_rank(RankLevel L, std::int32_t* __restrict__ p0,
+                                                   std::int32_t* __restrict__ p1, unsigned long long* __restrict__ err)
+{
+    LSDTT_COUNT();
+    extern __shared__ BlockNode node[];
+    const std::uint32_t n = min(*L.count, L.n), head = *L.head;
+    for (std::uint32_t v = threadIdx.x; v < n; v += 1024)
+    {
+        const std::uint32_t u = L.succ[v];
+        node[v] = BlockNode{u < n ? u : kEnd, L.w0[v], L.w1[v], 1u};
+    }
+    __syncthreads();
+    BlockNode own[kBlockPer];
+    for (int round = 0; round < 15; ++round)
+    {
+        bool more = false;
+#pragma unroll
+        for (int k = 0; k < kBlockPer; ++k)
+        {
+            const std::uint32_t v = k * 1024u + threadIdx.x;
+            if (k * 1024u >= n) break;  // (block-uniform)
+            if (v >= n) continue;
+            own[k] = node[v];
+            if (own[k].next != kEnd)
+            {
+                const BlockNode b = node[own[k].next];
+                own[k].next = b.next;
+                own[k].s0 += b.s0;
+                own[k].s1 += b.s1;
+                own[k].count += b.count;
+                more = true;
+            }
+        }
+        if (!__syncthreads_or(more)) break;
+#pragma unroll
+        for (int k = 0; k < kBlockPer; ++k)
+        {
+            const std::uint32_t v = k * 1024u + threadIdx.x;
+            if (k * 1024u >= n) break;
+            if (v < n) node[v] = own[k];
+        }
+        __syncthreads();
+    }
+    if (n == 0) return;
+    // One list from the head through every node, or the successors are not a
+    // list (a cycle never ends, a part beside it is not counted).
+    if (head >= n || node[head].next != kEnd || node[head].count != n)
+    {
+        if (threadIdx.x == 0) raise_error(err, kErrCycle, 2);
+        for (std::uint32_t v = threadIdx.x; v < n; v += 1024) p0[v] = p1[v] = 0;
+        return;
+    }
+    const std::int32_t t0 = node[head].s0, t1 = node[head].s1;
+    for (std::uint32_t v = threadIdx.x; v < n; v += 1024)
+    {
+        p0[v] = t0 - node[v].s0;
+        p1[v] = t1 - node[v].s1;
+    }
 }
 
 __global__ void serial_rank(RankLevel L, std::int32_t* __restrict__ p0, std::int32_t* __restrict__ p1,
@@ -428,14 +543,15 @@ __device__ __forceinline__ bool sv_masked(const SvOut& o, std::int64_t c)
 
 // rank_finish and sv_outputs in one pass over the cells of the level-0
 // (Euler tour) list: cell c's enter and exit records are adjacent.
-__global__ void sv_finish(RankLevel L, const RankRec* __restrict__ rec, const std::int32_t* __restrict__ P0,
+__global__ void sv_finish(RankLevel L, const TourRec* __restrict__ rec, const std::int32_t* __restrict__ P0,
                           const std::int32_t* __restrict__ P1, std::uint32_t cap, SvOut o,
                           unsigned long long* __restrict__ err)
 {
     LSDTT_COUNT();
     const std::int64_t c = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c >= o.g.n || sv_masked(o, c)) return;
-    const RankRec a = rec[2 * c], b = rec[2 * c + 1];
+    const uint4 q = reinterpret_cast<const uint4*>(rec)[c];
+    const TourRec a{q.x, q.y}, b{q.z, q.w};
     if (a.owner >= cap || b.owner >= cap)
     {
         // Not reached by any walk: the tour does not cover every valid node.
@@ -443,26 +559,62 @@ __global__ void sv_finish(RankLevel L, const RankRec* __restrict__ rec, const st
         sv_store(o, c, -1, -1, 0, err);
         return;
     }
-    sv_store(o, c, P0[a.owner] + a.loc0, P0[b.owner] + b.loc0, P1[a.owner] + a.loc1, err);
+    sv_store(o, c, P0[a.owner] + a.loc0(), P0[b.owner] + b.loc0(), P1[a.owner] + a.loc1(), err);
 }
 
 // Recursive list ranking. p0/p1 receive the exclusive prefix sums of the two
 // weights along the list starting at *L.head; with sv (the level-0 Euler
 // tour of a grid, longer than kSerialLimit) the per-cell s-vector outputs are
 // written instead and p0/p1 are not used.
+template <class Rec>
+cudaError_t rank_rulers(const RankLevel& L, std::int32_t* p0, std::int32_t* p1, Scratch& ws, unsigned long long* err,
+                        cudaStream_t st, const SvOut* sv);
+
 cudaError_t rank_list(const RankLevel& L, std::int32_t* p0, std::int32_t* p1, Scratch& ws,
                       unsigned long long* err, cudaStream_t st, const SvOut* sv = nullptr)
 {
+    if (sv) return rank_rulers<TourRec>(L, p0, p1, ws, err, st, sv);
     if (L.n <= static_cast<std::uint32_t>(kSerialLimit))
     {
         serial_rank<<<1, 32, 0, st>>>(L, p0, p1, err);
         return cudaGetLastError();
     }
+    if (L.n <= kBlockLimit && L.count)
+    {
+        const int bytes = static_cast<int>(sizeof(BlockNode) * L.n);
+        const cudaError_t e = cudaFuncSetAttribute(block_rank, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(sizeof(BlockNode) * kBlockLimit));
+        if (e != cudaSuccess) return e;
+        block_rank<<<1, 1024, bytes, st>>>(L, p0, p1, err);
+        return cudaGetLastError();
+    }
+    return rank_rulers<RankRec>(L, p0, p1, ws, err, st, nullptr);
+}
+
+void launch_finish(const RankLevel& L, const TourRec* rec, const std::int32_t* P0, const std::int32_t* P1,
+                   std::uint32_t cap, std::int32_t*, std::int32_t*, unsigned long long* err, cudaStream_t st,
+                   const SvOut* sv)
+{
+    sv_finish<<<grid_blocks(sv->g.n, 256), 256, 0, st>>>(L, rec, P0, P1, cap, *sv, err);
+}
+
+void launch_finish(const RankLevel& L, const RankRec* rec, const std::int32_t* P0, const std::int32_t* P1,
+                   std::uint32_t cap, std::int32_t* p0, std::int32_t* p1, unsigned long long* err, cudaStream_t st,
+                   const SvOut*)
+{
+    rank_finish<<<grid_blocks(L.n, 256), 256, 0, st>>>(L, rec, P0, P1, cap, p0, p1, err);
+}
+
+template <class Rec>
+cudaError_t rank_rulers(const RankLevel& L, std::int32_t* p0, std::int32_t* p1, Scratch& ws, unsigned long long* err,
+                        cudaStream_t st, const SvOut* sv)
+{
     const std::size_t mark = ws.used;
     const std::uint32_t cap = L.n / (kRuler / 4) + 64;  // generous bound on the ruler count
-    // cnt: [0] rulers, [1] the head's ruler, [2] valid nodes, [3] nodes walked
-    std::uint32_t* cnt = ws.take<std::uint32_t>(4);
-    RankRec* rec = ws.take<RankRec>(L.n);
+    // cnt: [0] rulers, [1] the head's ruler, [2] valid nodes, [3] nodes walked,
+    // [4] rulers that walks split off
+    std::uint32_t* cnt = ws.take<std::uint32_t>(5);
+    Rec* rec = ws.take<Rec>(L.n);
     // The ruler count is data dependent; size everything by `cap` and let the
     // kernels read the true count. A count above `cap` is reported.
     std::uint32_t* rulers = ws.take<std::uint32_t>(cap);
@@ -473,22 +625,17 @@ cudaError_t rank_list(const RankLevel& L, std::int32_t* p0, std::int32_t* p1, Sc
     std::int32_t* P1 = ws.take<std::int32_t>(cap);
     std::uint32_t* nhead = cnt + 1;
     if (!cnt || !rec || !rulers || !nxt || !sub0 || !sub1 || !P0 || !P1) return cudaErrorMemoryAllocation;
-    const unsigned nb = grid_blocks(L.n, 256);
-    cudaMemsetAsync(cnt, 0, sizeof(std::uint32_t) * 4, st);
-    ruler_compact<<<grid_blocks((L.n + kCompactPer - 1) / kCompactPer, 256), 256, 0, st>>>(L, cap, rulers, rec, cnt);
-    // Bytes touched per tour node: successor 4 in, the 16-byte record out.
-    LSDTT_TIMED("stack_ruler_walk", 20.0 * static_cast<double>(L.n), st,
-                (ruler_walk<<<grid_blocks(cap, 128), 128, 0, st>>>(L, rulers, cnt, rec, sub0, sub1, nxt, nhead,
-                                                                   cnt + 3, cap, err)));
+    cudaMemsetAsync(cnt, 0, sizeof(std::uint32_t) * 5, st);
+    ruler_compact<Rec>
+        <<<grid_blocks((L.n + kCompactPer - 1) / kCompactPer, 256), 256, 0, st>>>(L, cap, rulers, rec, cnt);
+    // Bytes touched per node: successor 4 in, the record out.
+    LSDTT_TIMED("stack_ruler_walk", (4.0 + sizeof(Rec)) * static_cast<double>(L.n), st,
+                (ruler_walk<Rec><<<grid_blocks(cap, 128), 128, 0, st>>>(L, rulers, cnt, rec, sub0, sub1, nxt, nhead, cap, err)));
     ruler_checks<<<1, 1, 0, st>>>(cnt, cap, err);
-    cudaError_t e = cudaSuccess;
     RankLevel up{cap, nxt, sub0, sub1, nullptr, nhead, cnt};
-    e = rank_list(up, P0, P1, ws, err, st);
+    const cudaError_t e = rank_list(up, P0, P1, ws, err, st);
     if (e != cudaSuccess) return e;
-    if (sv)
-        sv_finish<<<grid_blocks(sv->g.n, 256), 256, 0, st>>>(L, rec, P0, P1, cap, *sv, err);
-    else
-        rank_finish<<<nb, 256, 0, st>>>(L, rec, P0, P1, cap, p0, p1, err);
+    launch_finish(L, rec, P0, P1, cap, p0, p1, err, st, sv);
     ws.used = mark;
     return cudaGetLastError();
 }

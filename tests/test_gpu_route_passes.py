@@ -22,7 +22,9 @@ def _surface(nr, nc, kind, seed):
 CASES = [(1, 1, "oooo", "noise"), (1, 700, "oooo", "tilt"), (3000, 1, "oooo", "ramp"), (2, 2048, "opop", "noise"),
          (2048, 2, "popo", "noise"), (63, 65, "nnon", "noise"), (64, 64, "oooo", "noise"), (17, 241, "popo", "tilt"),
          (128, 96, "oooo", "mask"), (257, 160, "opop", "mask"), (301, 307, "nnon", "noise"), (600, 70, "oooo", "tilt"),
-         (1500, 3, "popo", "ramp"), (420, 400, "popo", "tilt")]
+         (1500, 3, "popo", "ramp"), (420, 400, "popo", "tilt"),
+         # the largest tour whose rulers one block ranks, and one row of cells more
+         (191, 256, "nnon", "noise"), (192, 256, "oooo", "tilt"), (700, 701, "nnon", "tilt")]
 
 
 @pytest.mark.parametrize("nr,nc,bc,kind", CASES)
