@@ -109,6 +109,14 @@ __global__ void __launch_bounds__(256) check_inputs(const float* __restrict__ z,
     }
 }
 
+// The engine's four error words: nothing raised, no first bad index (a copy from
+// pageable host memory holds the caller up for several microseconds).
+__global__ void reset_errors(unsigned long long* __restrict__ err)
+{
+    LSDTT_COUNT();
+    if (threadIdx.x < 4) err[threadIdx.x] = (threadIdx.x & 1u) ? ~0ull : 0ull;
+}
+
 __global__ void check_finite_w(const double* __restrict__ w, const std::uint8_t* __restrict__ mask, std::int64_t n,
                                unsigned long long* __restrict__ first_bad)
 {
@@ -348,8 +356,7 @@ int lsdtt_gpu_flow_build(lsdtt_gpu_flow* f, const float* z_dev, const std::uint8
     // validate_inputs (src/cpu/lsdtt_flowinfo_cpu.cpp:887-966): every valid
     // cell needs a finite, non-nodata elevation. derr[1] = first bad cell,
     // derr[3] = first bad forced-outlet entry.
-    unsigned long long init[4] = {0ull, ~0ull, 0ull, ~0ull};
-    cudaMemcpyAsync(f->derr, init, sizeof(init), cudaMemcpyHostToDevice, st);
+    reset_errors<<<1, 32, 0, st>>>(f->derr);
     check_inputs<<<grid_blocks(n, 256 * kInputPer), 256, 0, st>>>(z_dev, mask_dev, n, static_cast<float>(g.nodata),
                                                                   f->mask, f->derr + 1);
     std::uint8_t* plane = nullptr;
@@ -360,7 +367,7 @@ int lsdtt_gpu_flow_build(lsdtt_gpu_flow* f, const float* z_dev, const std::uint8
         stamp_forced<<<grid_blocks(n_forced, 256), 256, 0, st>>>(forced_dev, n_forced, n, f->mask, plane,
                                                                 f->derr + 3);
     }
-    cudaMemcpyAsync(f->herr, f->derr, sizeof(init), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(f->herr, f->derr, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "lsdtt_gpu_flow_build");
     if (f->herr[1] != ~0ull)
@@ -386,7 +393,7 @@ int lsdtt_gpu_flow_build(lsdtt_gpu_flow* f, const float* z_dev, const std::uint8
                                           std::to_string(fl % g.nc) +
                                           ") lands on a nodata or masked cell, so it cannot act as a flow termination");
     }
-    cudaMemcpyAsync(f->derr, init, sizeof(init), cudaMemcpyHostToDevice, st);
+    reset_errors<<<1, 32, 0, st>>>(f->derr);
 
     e = launch_receivers(f, z_dev, f->mask, plane, o.interior_nodata_is_outlet, o.allow_pits_as_outlets, st);
     if (e == cudaSuccess) e = launch_donors_outlets(f, st);
@@ -468,10 +475,9 @@ int lsdtt_gpu_flow_accumulate(lsdtt_gpu_flow* f, const double* w_dev, double* ou
     if (w_dev)
     {
         // cell_weights must be finite on every valid cell (:2001-2015).
-        unsigned long long init = ~0ull;
-        cudaMemcpyAsync(f->derr + 1, &init, sizeof(init), cudaMemcpyHostToDevice, st);
+        cudaMemsetAsync(f->derr + 1, 0xff, sizeof(unsigned long long), st);
         check_finite_w<<<grid_blocks(f->g.n, 256), 256, 0, st>>>(w_dev, f->mask, f->g.n, f->derr + 1);
-        cudaMemcpyAsync(f->herr + 1, f->derr + 1, sizeof(init), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(f->herr + 1, f->derr + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
         cudaError_t e0 = cudaStreamSynchronize(st);
         if (e0 != cudaSuccess) return cuda_fail(e0, "lsdtt_gpu_flow_accumulate");
         if (f->herr[1] != ~0ull)

@@ -701,13 +701,48 @@ __global__ void rmq_level(const std::uint64_t* __restrict__ prev, std::int64_t n
     next[b] = v;
 }
 
+// All levels of a small table (level k at base + k * stride; level 0 is there)
+// by one block, in shared memory: a launch a level took 2.5 us for nothing.
+constexpr int kRmqBlock = 4096;
+
+__global__ void __launch_bounds__(1024) rmq_levels(std::uint64_t* __restrict__ base, std::int64_t stride, int nb,
+                                                   int levels)
+{
+    LSDTT_COUNT();
+    __shared__ std::uint64_t t[kRmqBlock];
+    constexpr int kPer = kRmqBlock / 1024;
+    for (int b = threadIdx.x; b < nb; b += 1024) t[b] = base[b];
+    __syncthreads();
+    for (int k = 1; k < levels; ++k)
+    {
+        const int half = 1 << (k - 1);
+        std::uint64_t v[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j)
+        {
+            const int b = j * 1024 + threadIdx.x;
+            v[j] = b < nb ? t[b] : 0;
+            if (b + half < nb && t[b + half] > v[j]) v[j] = t[b + half];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; ++j)
+        {
+            const int b = j * 1024 + threadIdx.x;
+            if (b >= nb) continue;
+            t[b] = v[j];
+            base[k * stride + b] = v[j];
+        }
+        __syncthreads();
+    }
+}
+
 struct Rmq
 {
     const std::uint64_t* A;
     const std::uint64_t* pre;
     const std::uint64_t* suf;
-    const std::uint64_t* const* table;  // device array of level pointers
-    int levels;
+    const std::uint64_t* table[40];  // the levels, by value
 };
 
 __device__ std::uint64_t rmq_query(const Rmq& R, std::int64_t a, std::int64_t b)  // inclusive
@@ -880,14 +915,16 @@ cudaError_t build_stack(lsdtt_gpu_flow* f, bool want_topo, cudaStream_t st, cons
     std::uint64_t* suf = ws.take<std::uint64_t>(nv);
     int levels = 1;
     while ((std::int64_t(1) << levels) <= nblk) ++levels;
-    std::uint64_t* tab[40] = {};
-    for (int k = 0; k < levels; ++k) tab[k] = ws.take<std::uint64_t>(nblk);
-    std::uint64_t** dtab = ws.take<std::uint64_t*>(40);
-    if (!A || !pre || !suf || !dtab || !tab[levels - 1]) return cudaErrorMemoryAllocation;
-    rmq_base<<<grid_blocks(nblk * 32, 256), 256, 0, st>>>(f->svec, f->depth, nv, A, pre, suf, tab[0]);
-    for (int k = 1; k < levels; ++k)
-        rmq_level<<<grid_blocks(nblk, 256), 256, 0, st>>>(tab[k - 1], nblk, std::int64_t(1) << (k - 1), tab[k]);
-    cudaMemcpyAsync(dtab, tab, sizeof(tab), cudaMemcpyHostToDevice, st);
+    const std::int64_t stride = (nblk + 31) / 32 * 32;
+    std::uint64_t* tab = ws.take<std::uint64_t>(static_cast<std::size_t>(stride) * levels);
+    if (!A || !pre || !suf || !tab || levels > 40) return cudaErrorMemoryAllocation;
+    rmq_base<<<grid_blocks(nblk * 32, 256), 256, 0, st>>>(f->svec, f->depth, nv, A, pre, suf, tab);
+    if (nblk <= kRmqBlock)
+        rmq_levels<<<1, 1024, 0, st>>>(tab, stride, static_cast<int>(nblk), levels);
+    else
+        for (int k = 1; k < levels; ++k)
+            rmq_level<<<grid_blocks(nblk, 256), 256, 0, st>>>(tab + (k - 1) * stride, nblk, std::int64_t(1) << (k - 1),
+                                                              tab + k * stride);
 
     std::uint64_t* k0 = ws.take<std::uint64_t>(n);
     std::uint32_t* v0 = ws.take<std::uint32_t>(n);
@@ -896,7 +933,8 @@ cudaError_t build_stack(lsdtt_gpu_flow* f, bool want_topo, cudaStream_t st, cons
     std::uint32_t* leaf = ws.take<std::uint32_t>(n);
     if (!k0 || !v0 || !k1 || !v1 || !leaf) return cudaErrorMemoryAllocation;
     const int leaf_bits = bits_for(static_cast<std::uint64_t>(n - 1) | 1);
-    Rmq R{A, pre, suf, dtab, levels};
+    Rmq R{A, pre, suf, {}};
+    for (int k = 0; k < levels; ++k) R.table[k] = tab + k * stride;
     cudaMemsetAsync(f->derr + 2, 0, sizeof(unsigned long long), st);
     topo_heights<<<grid_blocks(n, 256 * kHeightPer), 256, 0, st>>>(g, f->mask, f->sv_start, f->sv_size, f->depth, R, f->height, leaf, f->derr + 2);
     // The number of radix passes depends on the tallest level: read it back.
