@@ -24,7 +24,11 @@ CASES = [(1, 1, "oooo", "noise"), (1, 700, "oooo", "tilt"), (3000, 1, "oooo", "r
          (128, 96, "oooo", "mask"), (257, 160, "opop", "mask"), (301, 307, "nnon", "noise"), (600, 70, "oooo", "tilt"),
          (1500, 3, "popo", "ramp"), (420, 400, "popo", "tilt"),
          # the largest tour whose rulers one block ranks, and one row of cells more
-         (191, 256, "nnon", "noise"), (192, 256, "oooo", "tilt"), (700, 701, "nnon", "tilt")]
+         (191, 256, "nnon", "noise"), (192, 256, "oooo", "tilt"), (700, 701, "nnon", "tilt"),
+         # the largest range-max table that one block builds, and a cell-row more
+         (512, 256, "oooo", "noise"), (513, 256, "nnon", "noise"),
+         # histograms of the sort scanned by one block (128 tiles), and past it
+         (512, 1024, "oooo", "noise"), (513, 1024, "oooo", "noise")]
 
 
 @pytest.mark.parametrize("nr,nc,bc,kind", CASES)
