@@ -354,9 +354,10 @@ __global__ void __launch_bounds__(32) ex_windows(const ExMember* __restrict__ me
     if (total < min_windows) return;  // (they stay marked as they are)
     for (;;)
     {
-        if (chain_done && *reinterpret_cast<const volatile unsigned*>(chain_done)) break;
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(work, 1u);
+        // (one lane reads the chain's word and decides for the warp)
+        unsigned t = total;
+        if (lane == 0 && !(chain_done && *reinterpret_cast<const volatile unsigned*>(chain_done)))
+            t = atomicAdd(work, 1u);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= total) break;
         const int g = wl[t];

@@ -1804,8 +1804,10 @@ __device__ int win_sweep_replay(const WinGrid& G, int w, const SweepBufs& B, flo
         int rounds = 0;
         for (;;)
         {
+            // (every thread has read the flag before a list of this round can
+            // overflow and set it)
             const std::uint32_t nch = min(sh.cnt[0], static_cast<std::uint32_t>(kSwL));
-            if (nch == 0 || sh.cnt[5]) break;
+            if (__syncthreads_or(nch == 0 || sh.cnt[5])) break;
             // a sweep settles in two or three rounds; one that has not after
             // 64 leaves the window to the sequential rules
             if (++rounds > 64)

@@ -467,10 +467,16 @@ __device__ WinResult win_replay(const WinGrid& G, int w, const WinStore& s, std:
                 }
             }
         }
-        if (quit && (pops & 31) == 31 && *reinterpret_cast<const volatile unsigned*>(quit))
+        if (quit && (pops & 31) == 31)
         {
-            res.status = kWinOverflow;
-            break;
+            // one lane reads the word: lanes that read it apart could disagree
+            unsigned gone = 0;
+            if (lane == 0) gone = *reinterpret_cast<const volatile unsigned*>(quit);
+            if (__shfl_sync(full, gone, 0))
+            {
+                res.status = kWinOverflow;
+                break;
+            }
         }
         if (pop_limit && ++pops > pop_limit)
         {
