@@ -191,7 +191,11 @@ __device__ __forceinline__ float4 sw_record(const float4* p)
 // first FIFO index >= g0 (1-based) whose value exceeds key; m + 1 if none
 __device__ __forceinline__ std::uint32_t sw_ng(const SweepShared& sh, std::uint32_t m, std::uint32_t g0, float key)
 {
-    std::uint32_t g = g0;
+    // (an event read while its cell's thread writes it can pair the sweep's
+    // stamp with a time of zero: gap 0, whose table entry does not exist and
+    // sent the search round for ever. The writer lists the cell, so the round
+    // after reads it whole.)
+    std::uint32_t g = max(g0, 1u);
     if (m <= kSwScan)
         while (g <= m && !(sh.fv[g - 1] > key)) ++g;
     else

@@ -52,3 +52,14 @@ def test_sweep_forms_bitwise(port, name, make, bc, cell, eps):
     differ = int((got.view(np.uint32) != want.view(np.uint32)).sum())
     print(f"{name}: {int((want != z).sum())} raised cells, {differ} differ")
     assert differ == 0
+
+
+def test_wide_sweeps_repeat(port):
+    """Noise at a slope whose sweeps outgrow the shared-memory forms: every call ends, with the same bits."""
+    import lsdtt_gb300 as G
+    z = (np.random.default_rng(5).random((160, 147)) + 0.03 * np.arange(159, -1, -1)[:, None]).astype(np.float32)
+    m = np.ones(z.shape, np.uint8)
+    want = port.fill_pits_index_ties(z, m, 30.0, "oooo", 1e-2).view(np.uint32)
+    for _ in range(150):
+        got = G.fill_pits(z, m, 30.0, "oooo", 1e-2).cpu().numpy().view(np.uint32)
+        assert int((got != want).sum()) == 0
