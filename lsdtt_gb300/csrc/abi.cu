@@ -292,8 +292,8 @@ int lsdtt_gpu_flow_create(const lsdtt_gpu_grid* grid, lsdtt_gpu_flow** out)
     alloc(&f->dscal, 4);
     alloc(&f->derr, 4);
     alloc(&f->dundec, 1);
-    // Workspace: the Euler-tour ranking peaks at ~60 B per cell (tour links
-    // 16 B, level-0 ruler records 32 B, the ruler lists and the upper
+    // Workspace: the Euler-tour ranking peaks at ~44 B per cell (tour links
+    // 16 B, level-0 ruler records 16 B, the ruler lists and the upper
     // levels; prefix arrays only for tours short enough for the serial
     // ranking); the range-max structure and the sort need ~58 B per cell
     // after the tour is released.
