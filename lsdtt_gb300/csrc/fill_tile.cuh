@@ -304,6 +304,8 @@ __device__ __forceinline__ void fill_relax_tile(int nr, int nc, bool per_ns, boo
 //
 // The maps are monotone and start from +inf, so the fixed point (the epsilon-0
 // fill, bit for bit) does not depend on the order in which tiles are relaxed.
+// (fmaxf and fminf order -0 below +0 and the rule does not: relax_fill takes a
+// surface with a -0 through the colours.)
 // A pass takes all its tiles in one launch, without colours, and a tile that
 // changed cells on its rim queues just the neighbours beyond them for the next
 // pass. 4099 x 4000 pitted fractal, wrapped: 24.0 ms in 696 launches, now 10.0
@@ -329,7 +331,7 @@ struct ScanTile
 struct TileQueue
 {
     std::int32_t* list[2];
-    unsigned* cnt;     // [3]
+    unsigned* cnt;     // [3] (and a flag of the caller's)
     unsigned* queued;  // [tiles]
 };
 
