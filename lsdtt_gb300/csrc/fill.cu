@@ -88,7 +88,7 @@ __global__ void fill_queue_init(int tiles, TileQueue Q)
 }
 
 // A pass over the queued tiles by a persistent grid (block w takes entries w,
-// w + grid, ...).
+// w + grid, ...). `pass`: its number modulo 6 (two lists and three counts in turn).
 template <bool kStep>
 __global__ void __launch_bounds__(256) fill_scan_pass(int nr, int nc, bool per_ns, bool per_ew, float L, float Ld,
                                                       float eps, const float* __restrict__ z,
@@ -117,6 +117,17 @@ using namespace lsdtt_gb300;
 namespace
 {
 
+// Passes between two looks at whether anything changed (to keep the host out of
+// the loop), and a bound on the passes that change a grid of n cells. A change in
+// a pass follows from a neighbour's change in that pass or the one before, whose
+// value is not above it. Back along such a chain values never rise, and a cell's
+// own values only fall, so a chain holds each cell once and no more than n
+// passes change anything. (A corridor that winds through the grid comes near
+// it: what counts is the tiles it crosses, some 6,400 in 640 x 640 cells with a
+// wall every second row.)
+constexpr int kCheckEvery = 4;
+inline std::int64_t relax_pass_limit(std::int64_t n) { return n + kCheckEvery; }
+
 // The relaxation from fill_init to its fixed point with raise step `eps` by
 // passes over the tiles' colours in turn, the same from run to run also where
 // values compare equal and differ in their bits. `flags`: interior nodata,
@@ -131,15 +142,13 @@ cudaError_t relax_coloured(int nr, int nc, bool per_ns, bool per_ew, float L, fl
     const std::int64_t ntiles = static_cast<std::int64_t>(ntx) * nty;
     const unsigned colours = fill_colour_mask(ntx, nty, per_ns, per_ew);
     const dim3 block(32, 8);
-    const int kCheckEvery = 4;
-    const long max_pass = 4L * (nr + nc) + 64;
     cudaMemsetAsync(flags, 0, sizeof(int) * 2, st);
     cudaMemsetAsync(dirty, 1, static_cast<std::size_t>(2 * ntiles), st);
     fill_interior_nodata<<<grid_blocks(n, 256), 256, 0, st>>>(nr, nc, z_dev, mask_dev, nodata, flags);
     fill_init<<<grid_blocks(n, 256), 256, 0, st>>>(nr, nc, per_ns, per_ew, z_dev, mask_dev, nodata, flags, F, kind,
                                                    nullptr);
     int changed = 0;  // pageable host word: the read-back allocates nothing
-    for (long pass = 0; pass <= max_pass;)
+    for (std::int64_t pass = 0; pass <= relax_pass_limit(n);)
     {
         cudaMemsetAsync(flags + 1, 0, sizeof(int), st);
         for (int k = 0; k < kCheckEvery; ++k, ++pass)
@@ -189,15 +198,12 @@ cudaError_t relax_fill(int nr, int nc, bool per_ns, bool per_ew, float L, float 
     fill_queue_init<<<grid_blocks(std::max(ntiles, 4), 256), 256, 0, st>>>(ntiles, Q);
     fill_init<<<grid_blocks(n, 256), 256, 0, st>>>(nr, nc, per_ns, per_ew, z_dev, mask_dev, nodata, flags, F, kind,
                                                    eps > 0.0f ? nullptr : Q.cnt + 3);
-    // Passes until the queue is empty; its counts are read back every few
-    // passes to keep the host out of the loop.
-    const int kCheckEvery = 4;
-    const long max_pass = 4L * (nr + nc) + 64;  // bound: any path crosses each tile row/column at most a few times
+    // Passes until the queue is empty.
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned grid = static_cast<unsigned>(std::min(ntiles, std::max(1, sms) * 6));
-    int pass = 0;
+    std::int64_t pass = 0;
     unsigned cnt[4] = {0, 0, 0, 0};
     while (e == cudaSuccess)
     {
@@ -215,10 +221,11 @@ cudaError_t relax_fill(int nr, int nc, bool per_ns, bool per_ew, float L, float 
             LSDTT_TIMED("fill_relax", bytes, st, ({
                             if (eps > 0.0f)
                                 fill_scan_pass<true><<<grid, 256, 0, st>>>(nr, nc, per_ns, per_ew, L, Ld, eps, z_dev, kind,
-                                                                           F, ntx, nty, Q, pass);
+                                                                           F, ntx, nty, Q, static_cast<int>(pass % 6));
                             else
                                 fill_scan_pass<false><<<grid, 256, 0, st>>>(nr, nc, per_ns, per_ew, L, Ld, 0.0f, z_dev,
-                                                                            kind, F, ntx, nty, Q, pass);
+                                                                            kind, F, ntx, nty, Q,
+                                                                            static_cast<int>(pass % 6));
                         }));
         }
         if (e != cudaSuccess) break;
@@ -233,7 +240,7 @@ cudaError_t relax_fill(int nr, int nc, bool per_ns, bool per_ew, float L, float 
             *converged = true;
             break;
         }
-        if (pass > max_pass) break;
+        if (pass > relax_pass_limit(n)) break;
     }
     return e;
 }
