@@ -34,10 +34,12 @@ namespace
 // there. Against one FP64 atomic a block on a single address (0.76 ns each at
 // the L2) or a one-block kernel after every pass (4.5 us of its own) this
 // leaves about a microsecond, and the sums are the same on every run.
-// Within a block a sum is carried in two FP32 words (error-free additions,
-// about 48 bits): a warp's FP64 addition holds this part's FP64 pipe for 16
+// Within a block an iteration's FP32 products are summed in two FP32 words (the
+// high words without error, the errors in plain FP32: about 40 bits over a
+// block's 2048 or 4096 cells, where FP32 within a warp and FP64 beyond would
+// hold about 22): a warp's FP64 addition holds this part's FP64 pipe for 16
 // cycles, and ten of them a warp and quantity cost 6 us of a 16 us pass over a
-// million cells.
+// million cells. The set-up, once a solve, sums in FP64.
 struct Sum2
 {
     float h = 0.0f, l = 0.0f;
@@ -169,7 +171,7 @@ __global__ void hs_dofs(Hs H, const std::uint8_t* __restrict__ mask, const std::
 // east and west edges the longest by far, 47 us of a pass on 2048 x 2051. The
 // passes now take 24 and 33 us there (about 8 of each the grid-wide sum's
 // chain of fence, arrival and last block) where the three untiled passes they
-// replace took 162: a solve of 80 iterations 14.2 -> 5.3 ms.
+// replace took 162: a solve of 80 iterations 14.3 -> 5.4 ms.
 constexpr int kHslTC = 128;  // columns of a set-up block
 
 struct Strip
@@ -241,10 +243,12 @@ __device__ __forceinline__ float hsl_invd(const HslArgs& A, unsigned cl)
     return !(cl & 1u) ? 0.0f : (f == 4 ? A.invd[4] : (f == 3 ? A.invd[3] : (f == 2 ? A.invd[2] : (f == 1 ? A.invd[1] : A.invd[0]))));
 }
 
-// Classes, b = -F (F = -(D/h^2) sum_f (z_nb - z_P), its sum and product carried
-// in two FP32 words each, so b is rounded once as from FP64), r = b, x = 0;
-// ||b||^2, r.D^-1 r, max |F|.
-__global__ void __launch_bounds__(256) hsl_setup(HslArgs A, float DA_lo, const std::uint8_t* __restrict__ chan,
+// Classes, b = -F (F = -(D/h^2) sum_f (z_nb - z_P)), r = b, x = 0; ||b||^2,
+// r.D^-1 r, max |F|. All in FP64, b rounded once: this runs once a solve, and
+// the squares decide when the solve stops (in FP32 they leave its range from
+// |F| = 1.8e19 on). It takes 0.16 of the 5.44 ms of a 2048 x 2051 solve more than
+// with b in two FP32 words and FP32 squares.
+__global__ void __launch_bounds__(256) hsl_setup(HslArgs A, const std::uint8_t* __restrict__ chan,
                                                  const float* __restrict__ z, std::uint8_t* __restrict__ cls,
                                                  float* __restrict__ r, float* __restrict__ x)
 {
@@ -253,8 +257,7 @@ __global__ void __launch_bounds__(256) hsl_setup(HslArgs A, float DA_lo, const s
     const int ntx = (H.nc + kHslTC - 1) / kHslTC;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int row = static_cast<int>(blockIdx.x / ntx) * 8 + w, c0 = static_cast<int>(blockIdx.x % ntx) * kHslTC;
-    Sum2 v[2];
-    float mh = 0.0f, ml = 0.0f;  // largest |b| before its rounding
+    double bb = 0.0, rz = 0.0, fin = 0.0;
     if (row < H.nr)
     {
 #pragma unroll
@@ -269,38 +272,34 @@ __global__ void __launch_bounds__(256) hsl_setup(HslArgs A, float DA_lo, const s
             float b = 0.0f;
             if (cl)
             {
-                const float zp = z[i];
-                float sh = 0.0f, sl = 0.0f;
+                const double zp = z[i];
+                double flux = 0.0;
 #pragma unroll
                 for (int f = 0; f < 4; ++f)
                 {
                     const std::int64_t j = (cl & 2u) ? i + static_cast<std::int64_t>(kDr[f]) * H.nc + kDc[f]
                                                      : hs_nb(H, A.mask, row, c, kDr[f], kDc[f]);
-                    // (d, e) = z_nb - z_P exactly, then added to (sh, sl)
-                    const float zj = z[j], d = zj - zp, t = d - zj, e = (zj - (d - t)) + (-zp - t);
-                    const float u = sh + d, q = u - sh;
-                    sl += ((sh - (u - q)) + (d - q)) + e;
-                    sh = u;
+                    flux += static_cast<double>(z[j]) - zp;
                 }
-                const float ph = A.DA * sh;
-                const float pl = fmaf(A.DA, sh, -ph) + (A.DA * sl + DA_lo * sh);
-                b = ph + pl;
-                const float bl = (ph - b) + pl;
-                const float ah = fabsf(b), al = b < 0.0f ? -bl : bl;
-                if (ah > mh || (ah == mh && al > ml))
-                {
-                    mh = ah;
-                    ml = al;
-                }
-                v[0].add(b * b);
-                v[1].add(b * (b * hsl_invd(A, cl)));
+                const double F = -H.DA * flux;
+                b = static_cast<float>(-F);
+                bb += F * F;
+                rz += static_cast<double>(b) * (b * hsl_invd(A, cl));
+                fin = fmax(fin, fabs(F));
             }
             r[i] = b;
         }
     }
     const unsigned nblk = gridDim.x;
-    block_atomic_max_nonneg(&A.S->finf, static_cast<double>(mh) + static_cast<double>(ml));
-    block_partials<2>(v, A.part, nblk);
+    block_atomic_max_nonneg(&A.S->finf, fin);
+    bb = block_reduce_d(bb, false);
+    rz = block_reduce_d(rz, false);
+    if (threadIdx.x == 0)
+    {
+        A.part[blockIdx.x] = bb;
+        A.part[nblk + blockIdx.x] = rz;
+        __threadfence();
+    }
     if (!last_block(&A.S->arrived, nblk)) return;
     double t[2];
     total_partials<2>(A.part, nblk, t);
@@ -499,8 +498,7 @@ extern "C" int lsdtt_gpu_hillslope_linear_implicit(const lsdtt_gpu_grid* grid, c
     A.max_iter = kMaxIt;
     cudaMemsetAsync(A.S, 0, sizeof(HsState), st);
     const unsigned nb = grid_blocks(n, 256);
-    hsl_setup<<<tiles8, 256, 0, st>>>(A, static_cast<float>(H.DA - static_cast<double>(A.DA)), is_channel_dev, z_dev, cls,
-                                      r, x);
+    hsl_setup<<<tiles8, 256, 0, st>>>(A, is_channel_dev, z_dev, cls, r, x);
     // Iterations in batches, each followed by one read of the state; a batch
     // launched past convergence returns at once.
     HsState S{};
