@@ -1464,7 +1464,7 @@ __global__ void k_loss_grad(const float* __restrict__ y, const float* __restrict
 // cores have no FP32 inputs). The forms that these replaced read every
 // operand from global memory once per multiplication: one gradient on
 // 512 x 512 took 8.70 ms with them (6.2 ms the weight gradients) and takes
-// 0.72 ms with these, forward pass included.
+// 0.73 ms with these, forward pass included.
 //
 // GS of four consecutive output channels at position q of an Hq x Wq input.
 template <int CO, bool UP>
@@ -1600,8 +1600,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_data(int Hq, int Wq, const float
 // Weight and bias gradients: block (split, tap) sums GS_tap x X over its
 // share of the positions, 8 x 8 (co, ci) accumulators a thread, the threads
 // that one copy of the (co, ci) plane leaves over taking other positions of
-// each 64-position stage (added at the end in a fixed tree). The splits'
-// partial sums go to part[split][parameter] and are added in split order by
+// each 64-position stage (added at the end in a fixed tree). Shares are a
+// multiple of 16 positions, so that few positions are no long run of one thread
+// either. The splits' partial sums go to part[split][parameter] and are added in split order by
 // k_bwd_w_sum, so the gradient has the same bits on every run.
 template <int CI, int CO, bool UP>
 __global__ void __launch_bounds__(256, 2) k_bwd_w(int Hq, int Wq, const float* __restrict__ g,
@@ -1621,7 +1622,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_w(int Hq, int Wq, const float* _
     const int co4 = 4 * (t / (CI / 8)), ci4 = 4 * (t % (CI / 8));  // channels co4.. and CO/2 + co4.., likewise ci
     const int tap = blockIdx.y, dy = tap / 3 - 1, dx = tap % 3 - 1;
     const int nq = Hq * Wq;
-    const int len = ((nq + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + TQ - 1) / TQ * TQ;
+    const int len = ((nq + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + 15) / 16 * 16;
     const int qa = min(nq, static_cast<int>(blockIdx.x) * len), qb = min(nq, qa + len);
     float4 rg[NG];
     uint4 rx[NX];
@@ -1839,7 +1840,9 @@ __global__ void __launch_bounds__(256) k_bwd_data_out(int H, int W, const float*
                                                        m1.x > 0.f ? s.z : 0.f, m1.y > 0.f ? s.w : 0.f);
 }
 
-// Every parameter's gradient from its layer's partial sums, in split order.
+// Every parameter's gradient from its layer's partial sums, in split order, the
+// additions' errors carried along: up to 128 plain additions left 0.8-1.7e-7 of a
+// tensor's root mean square against 64 bits, these 0.3e-7 (512 x 512, 9 us more).
 struct WgradSplits
 {
     std::int64_t woff[kLayers + 1], boff[kLayers + 1];
@@ -1855,10 +1858,15 @@ __global__ void __launch_bounds__(256) k_bwd_w_sum(std::int64_t nparam, WgradSpl
     const std::int64_t* off = j < S.woff[kLayers] ? S.woff : S.boff;
     int l = 0;
     while (l + 1 < kLayers && j >= off[l + 1]) ++l;
-    float v = 0.f;
+    float h = 0.f, e = 0.f;
 #pragma unroll 8
-    for (int k = 0; k < S.splits[l]; ++k) v += part[k * nparam + j];
-    g[j] = v;
+    for (int k = 0; k < S.splits[l]; ++k)
+    {
+        const float v = part[k * nparam + j], t = h + v, q = t - h;
+        e += (h - (t - q)) + (v - q);
+        h = t;
+    }
+    g[j] = h + e;
 }
 
 __global__ void k_adam(std::int64_t n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
