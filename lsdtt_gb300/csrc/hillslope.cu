@@ -206,16 +206,6 @@ struct Strip
     }
 };
 
-// Blocks of a strip pass.
-inline unsigned strip_blocks(int nr, int nc, int rw)
-{
-    const std::int64_t g = static_cast<std::int64_t>((nc + 29) / 30) * ((nr + rw - 1) / rw);
-    return static_cast<unsigned>((g + 7) / 8);
-}
-// Rows a warp walks: 16 where that leaves every SM 32 warps (two halo rows in
-// 18 loaded, not two in 10), else 8.
-inline bool strip_long(int nr, int nc) { return strip_blocks(nr, nc, 16) >= 4 * 152; }
-
 struct HsState
 {
     double bb, rz, rr, rel, finf;
@@ -731,17 +721,13 @@ __global__ void hsn_pcg_init(HsN P, const std::uint8_t* __restrict__ mask, const
     block_atomic_add(&acc[1], bb);
 }
 
-// ---- tiled operator and fixed-order reductions of the PCG loops ------------
-// The loops below run the operator over 128 x 32 tiles with the direction
-// (or the network's output) staged in shared memory with a one-cell halo,
-// write one partial per block instead of atomics on a single address, and
-// reduce the partials in one block in a fixed order, which also forms alpha
-// or beta once (FP64 on this part is a narrow pipe: one division per block
-// stalled every block behind its thread 0).
-constexpr int kHsTC = 128, kHsTR = 32;
-constexpr int kHsUpdBlocks = 152 * 8;  // grid of the grid-stride update kernels
-
-inline int hs_tiles(int nr, int nc) { return ((nc + kHsTC - 1) / kHsTC) * ((nr + kHsTR - 1) / kHsTR); }
+// ---- operator and fixed-order reductions of the PCG loops -------------------
+// The loops below run the operator over strips and the learned
+// preconditioner's smoothing over 128 x 32 tiles (the network's output staged
+// in shared memory with a one-cell halo), write one partial per block (HsParts)
+// instead of atomics on a single address, and add the partials in a fixed
+// order in one block, which also forms alpha or beta once (FP64 on this part is
+// a narrow pipe: one division per block stalled every block behind its thread 0).
 
 // FP32 sum over the warp (lane 0 gets it; 32 terms, as block_atomic_add_f).
 __device__ __forceinline__ float warp_sum_f(float v)
@@ -1224,7 +1210,7 @@ struct HsnBuf
     float4* alpha;
     float *invd, *b, *x, *r, *p, *zz, *Ap, *ro;
     float* p2;     // the other direction buffer of the fused apply
-    double* part;  // block partials: 4 x tiles, then 2 x kHsUpdBlocks
+    double* part;  // block partials (HsParts)
     float* scal;   // [0] alpha, [1] beta of the current iteration
     HsnLoop* loop; // the loop's state, in the same 256 bytes
     double* hacc;
@@ -1236,8 +1222,7 @@ inline std::size_t hsn_pcg_bytes(int nr, int nc)
 {
     const std::size_t n = static_cast<std::size_t>(nr) * nc;
     return (4 * n + 255) / 256 * 256 +
-           (sizeof(double) * (4 * static_cast<std::size_t>(hs_tiles(nr, nc)) + 2 * kHsUpdBlocks) + 255) / 256 * 256 +
-           256;
+           (sizeof(double) * hs_parts(nr, nc).total + 255) / 256 * 256 + 256;
 }
 
 template <class Carve>
@@ -1245,8 +1230,7 @@ void hsn_pcg_carve(HsnBuf& B, int nr, int nc, Carve carve)
 {
     const std::size_t n = static_cast<std::size_t>(nr) * nc;
     B.p2 = reinterpret_cast<float*>(carve(4 * n));
-    B.part = reinterpret_cast<double*>(
-        carve(sizeof(double) * (4 * static_cast<std::size_t>(hs_tiles(nr, nc)) + 2 * kHsUpdBlocks)));
+    B.part = reinterpret_cast<double*>(carve(sizeof(double) * hs_parts(nr, nc).total));
     B.scal = reinterpret_cast<float*>(carve(256));
     B.loop = reinterpret_cast<HsnLoop*>(B.scal + 16);
 }
@@ -1285,11 +1269,11 @@ cudaError_t jacobi_loop(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::
                         double* rel, const std::vector<int>* snap_at = nullptr, float* x_snap = nullptr,
                         float* r_snap = nullptr, bool check = true)
 {
-    const int tiles = hs_tiles(P.H.nr, P.H.nc);
     const float inv_dt = static_cast<float>(P.H.inv_dt), DA = static_cast<float>(P.H.DA);
     float* pbuf[2] = {B.p, B.p2};
-    double* part_ap = B.part;
-    double* part_up = B.part + 4 * static_cast<std::size_t>(tiles);
+    const HsParts parts = hs_parts(P.H.nr, P.H.nc);
+    double* part_ap = B.part + parts.ap;
+    double* part_up = B.part + parts.up;
     const bool tall = strip_long(P.H.nr, P.H.nc);
     const unsigned nt = strip_blocks(P.H.nr, P.H.nc, tall ? 16 : 8);
     const unsigned ub = static_cast<unsigned>(std::min<std::int64_t>(kHsUpdBlocks, (n + 1023) / 1024));
@@ -1396,11 +1380,12 @@ cudaError_t hsn_pcg(const HsN& P, const std::uint8_t* mask, HsnBuf& B, std::int6
     const int tiles = hs_tiles(H, W);
     const float inv_dt = static_cast<float>(P.H.inv_dt), DA = static_cast<float>(P.H.DA);
     float* pbuf[2] = {B.p, B.p2};
-    double* part_ap = B.part;
-    double* part_rz = B.part + tiles;
-    double* part_roz = B.part + 2 * static_cast<std::size_t>(tiles);
+    const HsParts parts = hs_parts(H, W);
+    double* part_ap = B.part + parts.ap;
+    double* part_rz = B.part + parts.rz;
+    double* part_roz = B.part + parts.roz;
     const unsigned nt = strip_blocks(H, W, 8);
-    double* part_rr = B.part + 4 * static_cast<std::size_t>(tiles);
+    double* part_rr = B.part + parts.up;
     // z = y + D^-1 (r - A y), y = the network applied to q = D^-1 r (in zz),
     // masked to the DOFs; partials of r.z and z.(r - r_old)
     auto precondition = [&]() -> cudaError_t {

@@ -44,6 +44,38 @@ __device__ __forceinline__ bool hs_dirichlet_edge(const Hs& H, int r, int c)
            (c == H.nc - 1 && H.be == 'o');
 }
 
+// ---- shapes of the single-grid solvers' passes -------------------------------
+// Blocks of a strip pass.
+inline unsigned strip_blocks(int nr, int nc, int rw)
+{
+    const std::int64_t g = static_cast<std::int64_t>((nc + 29) / 30) * ((nr + rw - 1) / rw);
+    return static_cast<unsigned>((g + 7) / 8);
+}
+// Rows a warp walks: 16 where that leaves every SM 32 warps (two halo rows in
+// 18 loaded, not two in 10), else 8.
+inline bool strip_long(int nr, int nc) { return strip_blocks(nr, nc, 16) >= 4 * 152; }
+
+// Tiles of the learned preconditioner's smoothing, and the grid of the
+// grid-stride update kernels.
+constexpr int kHsTC = 128, kHsTR = 32;
+constexpr int kHsUpdBlocks = 152 * 8;
+
+inline int hs_tiles(int nr, int nc) { return ((nc + kHsTC - 1) / kHsTC) * ((nr + kHsTR - 1) / kHsTR); }
+
+// Where the Roering solver's block partials lie (doubles): p.Ap (a strip pass,
+// 8 rows at least), r.z and z.(r - r_old) (the smoothing), and the updates' two.
+struct HsParts
+{
+    std::size_t ap, rz, roz, up, total;
+};
+
+inline HsParts hs_parts(int nr, int nc)
+{
+    const std::size_t strips = strip_blocks(nr, nc, 8), tiles = static_cast<std::size_t>(hs_tiles(nr, nc));
+    const std::size_t up = strips + 2 * tiles;
+    return HsParts{0, strips, strips + tiles, up, up + 2 * kHsUpdBlocks};
+}
+
 __device__ constexpr int kDr[4] = {-1, 0, 1, 0};  // N, E, S, W
 __device__ constexpr int kDc[4] = {0, 1, 0, -1};
 
