@@ -105,7 +105,11 @@ int lsdtt_gpu_selftest_mbarrier_wait(int32_t tries);
  * equal value are taken in (row, col) order where the reference's heap
  * layout decides. Errors: LSDTT_GPU_EINVAL (arguments), LSDTT_GPU_ETIMEOUT
  * (the relaxation did not converge), LSDTT_GPU_EOVERFLOW (a window replay
- * outgrew its arrays). */
+ * outgrew its arrays).
+ * With min_slope > 0 a call makes a stream of its own (and two events) and
+ * destroys it before it returns: one thread block follows the fill's order on
+ * the caller's stream while replays ahead of it take up to every SM on the other.
+ * Kernels on a caller's further streams then run beside them more slowly. */
 int lsdtt_gpu_fill_pits(const lsdtt_gpu_grid* grid, const float* z_dev, const uint8_t* mask_dev,
                         float min_slope, float* filled_dev, void* stream);
 
@@ -119,7 +123,7 @@ int lsdtt_gpu_fill_pits(const lsdtt_gpu_grid* grid, const float* z_dev, const ui
  * at min_slope <= 0 and, because the raised cells' reference order needs
  * about 240 bytes a cell of replay buffers, about 520 x 520 cells at
  * min_slope > 0; larger grids return LSDTT_GPU_EINVAL. Same results as
- * lsdtt_gpu_fill_pits. It is never capturable: every call reads flags back
+ * lsdtt_gpu_fill_pits; everything runs on the given stream. It is never capturable: every call reads flags back
  * to the host between passes, and a call on a stream that is capturing
  * returns LSDTT_GPU_EINVAL before it enqueues anything. All calls share the
  * array, so calls that overlap on the GPU race; order them on one stream. */
@@ -252,6 +256,9 @@ int lsdtt_gpu_stream_power_d8(lsdtt_gpu_flow* flow, const float* z_dev, const fl
  * step of compute_hillslope_newton (src/cpu/lsdtt_hillslope_newton_cpu.cpp:
  * 196-675; operator src/cpu/lsdtt_hillslope_operator_cpu.hpp:83-322) with
  * alpha = 1, solved matrix-free by Jacobi-PCG to ||r||_2 <= rel_tol*||b||_2.
+ * The residual b and its norms are FP64; the iterations hold their vectors in
+ * FP32, form products in FP32 and add them in two FP32 words within a block and
+ * in FP64 across blocks.
  * is_channel_dev may be NULL (no channel cells). Returns LSDTT_GPU_ENOCONV
  * (with z_out still written) when max_iter is reached first. */
 typedef struct lsdtt_gpu_solve_report

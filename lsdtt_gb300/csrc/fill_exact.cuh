@@ -591,7 +591,9 @@ constexpr unsigned kExMinWindows = 20;
 // Pops after which the small size leaves a window to the replays beside the
 // chain, which waits for the small size only. (32, 96, 192, no limit: a
 // 97 x 131 noise tilt 3.18, 3.24, 3.36, 3.74 ms, a 1500 x 1403 pitted fractal
-// 152.7, 153.4, 153.2, 154.3.)
+// 152.7, 153.4, 153.2, 154.3. Larger grids do not tell: 32, 192, no limit on a
+// 3000 x 2900 fractal 669, 671, 671 ms, on an LEM surface of 512 x 512 9.0, 9.1,
+// 9.3, of 1024 x 1024 72.0, 72.2, 72.4, of 2048 x 2048 311 each.)
 constexpr unsigned long long kExSidePops = 32;
 constexpr std::size_t kExSmemA = 8 * kExA_FQ + 8 * (kExA_DH + 2) + 4 * kExA_HS + 8 * kExA_OC;
 constexpr std::size_t kExSmemM = 8 * kExM_FQ + 8 * (kExM_DH + 2) + 4 * kExM_HS + 8 * kExM_OC;
@@ -711,12 +713,15 @@ inline cudaError_t ex_run(const ExMember* mem, const std::uint16_t* blk_member, 
     // member per SM or more, the chains' block sweeps replay the windows the
     // small size could not hold -- only those on a chain, where the larger
     // sizes replay every such candidate one pop at a time -- and the step
-    // is faster without them (256 members: 358 ms a step with them, 234 ms
-    // without; one 2048 x 2048 grid: 498 ms with them, 779 ms without).
-    // A single grid's chain is one block: with `side` the larger sizes run
-    // beside it on the other SMs. The chain takes what they have finished when
-    // it gets there and replays the rest itself, and they stop when it is
-    // done; whichever replays a window, its raised cells are the same.
+    // is faster without them (256 members: 311 ms a step with them, 162
+    // without). A single grid's chain is one block: with `side` the larger
+    // sizes run beside it on the other SMs. The chain takes what they have
+    // finished when it gets there and replays the rest itself, and they stop
+    // when it is done; whichever replays a window, its raised cells are the
+    // same. (Beside the chain, before it, not at all: a 97 x 131 noise tilt 2.1,
+    // 2.7, 4.0 ms, an LEM surface of 512 x 512 8.9, 10.2, 30.3, of 2048 x 2048 311,
+    // 322, 312, a pitted fractal of 1500 x 1403 148, 157, 187, of 3000 x 2900 669,
+    // 682, 730.)
     auto larger = [&](cudaStream_t s, unsigned min_windows, const unsigned* done) {
         LSDTT_TIMED(nm[5], 16.0 * cells, s,
                     (ex_overflow_list<<<nb, 256, 0, s>>>(N, B.wl, B.u + 1, B.wl2, B.u + 3, B.status),

@@ -26,7 +26,8 @@
 // they reach in shared memory and read one record per (pop, direction); wide
 // ones keep one 16-byte event record per cell in global memory. With the wide
 // form alone a 1500 x 1403 pitted fractal filled in 329 ms (21,705 sweeps)
-// and a 256-member ensemble step took 241 ms; with the three, 163 and 186 ms.
+// and a 256-member ensemble step took 241 ms; with the three, 163 and 186 ms
+// (148 and 171 with what has changed around them since).
 #pragma once
 
 #include <cstdint>

@@ -308,17 +308,17 @@ __device__ __forceinline__ void fill_relax_tile(int nr, int nc, bool per_ns, boo
 // surface with a -0 through the colours.)
 // A pass takes all its tiles in one launch, without colours, and a tile that
 // changed cells on its rim queues just the neighbours beyond them for the next
-// pass. 4099 x 4000 pitted fractal, wrapped: 24.0 ms in 696 launches, now 10.0
-// in 140.
+// pass. 4099 x 4000 pitted fractal, wrapped: 24.0 ms in 696 launches, now about
+// 10 in 130 to 140.
 //
 // With a raise step the tile runs the four-colour rounds of fill_relax_tile
 // (a cell above its lowest neighbour keeps its elevation, however little: a
 // rule without a composed form, and rounding it up to one merged the windows
 // of LEM surfaces into a few long ones, 16 times the time of a step), queued
 // the same way: 512 x 512 LEM surface 1.43 ms, now 0.64 with the step-0 pass;
-// 1500 x 1403 fractal 6.5 ms, now 3.1. Its fixed point then depends on the schedule where the
-// discoverer rule is not monotone; it is only the estimate that chooses window
-// starts (fill_window.cuh), never a result.
+// 1500 x 1403 fractal 6.5 ms, now 3.1. Its fixed point then depends on the
+// schedule where the discoverer rule is not monotone; it is only the estimate
+// that chooses window starts (fill_window.cuh), never a result.
 struct ScanTile
 {
     float F[kH][kH + 1];
